@@ -370,7 +370,12 @@ struct NormalMomentLoad {
 
 // Node records from topology + moments + cell geometry (NodeRec, 80 B).
 // The topology fields were written by emit_nodes_kernel into nodes[k].topo.
-__global__ void finalize_nodes_kernel(NodeRec* __restrict__ nodes, const uint32_t* __restrict__ nn_ptr,
+// A node's children are the pre-order chain k + 1, skip(k + 1), ... inside its
+// subtree; their indices go to child[] so the walks open a node with two
+// 16-byte loads. (Other threads rewrite the records meanwhile, but never
+// their topology, so the skip fields read here are final.)
+__global__ void finalize_nodes_kernel(NodeRec* __restrict__ nodes, int4* __restrict__ child,
+                                      const uint32_t* __restrict__ nn_ptr,
                                       const uint64_t* __restrict__ keys, const uint32_t* __restrict__ sseg,
                                       const SegBox* __restrict__ boxes, const DVec<10>* __restrict__ P,
                                       const DVec<3>* __restrict__ PN, float4* __restrict__ nnrm) {
@@ -417,8 +422,26 @@ __global__ void finalize_nodes_kernel(NodeRec* __restrict__ nodes, const uint32_
     r.quad = make_float4(static_cast<float>(S[0]), static_cast<float>(S[1]), static_cast<float>(S[2]),
                          static_cast<float>(S[3]));
     r.quad2 = make_float4(static_cast<float>(S[4]), static_cast<float>(S[5]), 0.0f, 0.0f);
-    r.topo = t;
-    nodes[k] = r;
+    nodes[k].com = r.com;
+    nodes[k].cell = r.cell;
+    nodes[k].quad = r.quad;
+    nodes[k].quad2 = r.quad2;
+    if (!(t.w & kLeafFlag)) {
+      int c[8];
+      uint32_t j = k + 1;
+      const uint32_t end = static_cast<uint32_t>(t.z) < nn ? static_cast<uint32_t>(t.z) : nn;
+#pragma unroll
+      for (int i = 0; i < 8; i++) {
+        const bool in = j < end;
+        c[i] = in ? static_cast<int>(j) : -1;
+        if (in) {
+          const uint32_t s = static_cast<uint32_t>(nodes[j].topo.z);
+          j = s > j ? s : end;  // malformed skip: no further children
+        }
+      }
+      child[2 * static_cast<int64_t>(k)] = make_int4(c[0], c[1], c[2], c[3]);
+      child[2 * static_cast<int64_t>(k) + 1] = make_int4(c[4], c[5], c[6], c[7]);
+    }
     if (nnrm && PN) {
       DVec<3> nh = PN[e0], nl = PN[s0];
       nnrm[k] = M != 0.0 ? make_float4(static_cast<float>((nh.v[0] - nl.v[0]) / M),
@@ -564,6 +587,7 @@ __global__ void single_offsets_kernel(int64_t* seg_off, int64_t n) {
 // ---------------------------------------------------------------------------
 struct WalkTree {
   const NodeRec* nodes;
+  const int4* child;    // per node: its children's indices in order (8, unused slots -1), two int4
   const float4* sp;     // sorted sources (x, y, z, m)
   const float4* sn;     // sorted source normals (winding number)
   const float4* nnrm;   // node mean normals (winding number)
@@ -679,7 +703,7 @@ __device__ __forceinline__ void lq_symv(const float* A, float x0, float x1, floa
 // a_q(x) and J(x) packed, for x = c - X (the second moment S packed).
 __device__ __forceinline__ void lq_field(const float* x, const float* S, float eps2, float* a, float* J, float* f) {
   const float h = fmaf(x[0], x[0], fmaf(x[1], x[1], fmaf(x[2], x[2], eps2)));
-  const float ir = rsqrtf(h), ih = ir * ir;
+  const float ir = vrsqrt(h), ih = ir * ir;
   f[0] = ir * ih * ih;  // f2
   f[1] = f[0] * ih;     // f3
   f[2] = f[1] * ih;     // f4
@@ -744,28 +768,7 @@ __device__ __forceinline__ void lq_node_adjoint(const float* x, const float* S, 
   }
 }
 
-// ---------------------------------------------------------------------------
-// Node tiles staged in shared memory. The walks visit nodes in pre-order, so
-// after an opened node the next one is its neighbour in memory, and an
-// accepted node with a small subtree skips only a few records. A warp stages
-// the opening data (topology, COM, cell) of 32 consecutive nodes at once, one
-// node per lane, with cp.async (16 bytes a copy, cached in L2 only), and
-// walks from shared memory until the pre-order index leaves the tile. One L2
-// round trip then serves every visit inside the tile, where each visit used
-// to wait on its own loads. When a visit's successor lies outside the tile,
-// the next tile's copy starts before the visit's terms are evaluated and is
-// waited for only after them, so the copy overlaps the arithmetic.
-constexpr int kTile = 32;
-struct NodeTile {
-  int4 topo[kTile];
-  float4 com[kTile];
-  float4 cell[kTile];
-};
-
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-  const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
-}
+constexpr int kTile = 32;  // node records staged at once (the stochastic kernels)
 
 // Bulk copies (the TMA unit's non-tensor cp.async.bulk, no multicast) into
 // shared memory, completed on an mbarrier. The waits are bounded: a copy
@@ -806,37 +809,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t phase) {
   return false;
 }
 
-// Starts staging nodes [base, min(base + kTile, end)) into the warp's tile.
-// Every lane calls it (warp-uniform) after it has read what it needs from
-// the previous tile; stage_wait() completes the copy for all lanes.
-__device__ __forceinline__ void stage_tile_async(const NodeRec* __restrict__ nodes, int base, int end,
-                                                 NodeTile* tile, int lane) {
-  __syncwarp();  // every lane has finished reading the previous tile
-  const int k = base + lane;
-  if (k < end) {
-    const NodeRec* nd = nodes + k;
-    cp_async16(&tile->topo[lane], &nd->topo);
-    cp_async16(&tile->com[lane], &nd->com);
-    cp_async16(&tile->cell[lane], &nd->cell);
-  }
-  asm volatile("cp.async.commit_group;\n" ::: "memory");
-}
-
-__device__ __forceinline__ void stage_wait() {
-  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-  __syncwarp();
-}
-
-// Per-warp shared state of the linearized quadrupole during one group's walk:
-// the queue of accepted nodes waiting for their one-per-group evaluation (one
-// node per lane when 32 have gathered), each lane's running sums of a_q and
-// J over the nodes it evaluated, and the group's constants.
-struct LinQueue {
-  int node[32];
-  float acc[9][32];  // [a_q (3), J (6)][lane]
-  float grp[16];     // c (3), r_g^2, W (3), V (6)
-};
-
 // Group centre and squared half diagonal, IEEE operations in the oracle's
 // order (group_centre in oracle/sbh_oracle.c), so both take the same
 // linearization decisions.
@@ -864,75 +836,211 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
-// Evaluates the queued nodes, one per lane (lanes < cnt): adds a_q and J to
-// the lane's sums and, when node_adj is given, the node's dL/dX and dL/dS.
-__device__ __forceinline__ void lq_flush(const NodeRec* __restrict__ nodes, LinQueue* lq, int cnt, float eps2,
-                                         float* __restrict__ node_adj, int lane) {
-  __syncwarp();
-  if (lane < cnt) {
-    const int k = lq->node[lane];
-    const NodeRec* nd = nodes + k;
-    const float4 A = __ldg(&nd->com), Qd = __ldg(&nd->quad), X2 = __ldg(&nd->quad2);
-    const float x[3] = {lq->grp[0] - A.x, lq->grp[1] - A.y, lq->grp[2] - A.z};
-    const float S[6] = {Qd.x, Qd.y, Qd.z, Qd.w, X2.x, X2.y};
-    float a[3], J[6], f[4];
-    lq_field(x, S, eps2, a, J, f);
-#pragma unroll
-    for (int c = 0; c < 3; c++) lq->acc[c][lane] += a[c];
-#pragma unroll
-    for (int c = 0; c < 6; c++) lq->acc[3 + c][lane] += J[c];
-    if (node_adj) {
-      float g[3], G[6];
-      lq_node_adjoint(x, S, J, f, &lq->grp[4], &lq->grp[7], g, G);
-      float* na = node_adj + static_cast<int64_t>(k) * kNodeAdj;
-#pragma unroll
-      for (int c = 0; c < 3; c++) atomicAdd(&na[c], -g[c]);
-#pragma unroll
-      for (int c = 0; c < 6; c++) atomicAdd(&na[4 + c], G[c]);
-    }
-  }
-  __syncwarp();
+// Vector reductions to global memory (16- and 8-byte aligned).
+__device__ __forceinline__ void red_add4(float* p, float a, float b, float c, float d) {
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
+__device__ __forceinline__ void red_add2(float* p, float a, float b) {
+  asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(p), "f"(a), "f"(b) : "memory");
 }
 
-// The walks are compiled three times: four targets per lane (groups of up
-// to 128), three (up to 96) and two (up to 64), each for the occupancy that
-// suits it. Measured on a
-// B200 over 8 x 2^20 Plummer particles at quadrupole radius 1.6, the adjoint
-// walk takes 410 ms with two targets per lane at 7 blocks per SM (72
-// registers) and 389 ms with three at 6 blocks (80 registers); 4 per lane at
-// 4 blocks takes 411 ms. The adjoint walk's packed form (two slots per FP32
-// instruction) then brought three per lane to 367 ms at 5 blocks (96
-// registers), against 374 ms for the scalar form at 6 blocks and 397 ms at 5;
-// packed at 4 blocks it takes 403 ms. Two per lane packed stays best at 7
-// blocks (the 2^21 lattice walk: 33.9 ms, 34.8 at 6, 36.9 at 5; scalar 36.9
-// at 7). Four per lane packed (two full pairs, groups of 128) at 4 blocks
-// (128 registers) takes 356 ms; its force walk at 5 blocks (102 registers)
-// builds + forces one 2^20 Plummer system in 22.7 ms (23.2 at 4 blocks, 24.1
-// with groups of 96). Clustered systems gain from the
-// larger groups;
-// near-uniform ones and walks bounded by a prune radius gain from smaller
-// groups (a 2^21 lattice trajectory: 3.76 s with groups of 64, 4.46 s with
-// 96), which the two-slot kernels serve. A tree walks with the kernels of its
-// current group size (sbh_native_set_group_size).
+// ---------------------------------------------------------------------------
+// Shared state of a walk by W cooperating warps (see sbh_native_walks.inc).
+// ---------------------------------------------------------------------------
+template <int N>
+struct SlotCount {
+  static constexpr int value = N;
+};
+
+// Frontier and work lists of one group. A step adds at most 32 W entries to
+// each list and the lists are served in batches of 32 W as soon as they hold
+// that many, so 64 W entries suffice.
+template <int W>
+struct WalkQueues {
+  static constexpr int kStack = 512 + 256 * W;
+  int stack[kStack];
+  int far[64 * W];    // accepted nodes (negative: with the linearized quadrupole)
+  int quad[64 * W];   // accepted nodes with the exact quadrupole
+  int2 leaf[64 * W];  // near leaves: first particle, count
+  int4 cnt[W];        // one step's additions per warp (far, quad, leaf, stack)
+  float box[12];      // group box: minima, maxima; its centre and squared half diagonal
+  uint32_t group;
+};
+
+// One warp's share: the staged sources of its batch, their indices, its sums
+// of the linearized quadrupoles (a_q (3), J (6) per lane) and, for the
+// adjoint, the group's cotangent sums (W (3), V (6)) and the reduction buffer.
+constexpr int kRedStride = 36;  // float4 per row: 32 lanes, padded so four lanes' reads of eight rows miss each other's banks
+template <bool ADJ>
+struct WarpShared {
+  float4 stage[96];
+  int idx[32];
+  float acc[9][32];
+};
+template <>
+struct WarpShared<true> {
+  float4 stage[96];
+  float4 red[8 * kRedStride];
+  int idx[32];
+  float acc[9][32];
+  float wv[12];
+};
+
+template <int W, bool ADJ>
+struct __align__(16) CoopShared {
+  WarpShared<ADJ> w[W];
+  WalkQueues<W> q;
+};
+
+template <int W>
+__device__ __forceinline__ uint32_t coop_next_group(const WalkTargets& G, WalkQueues<W>& q) {
+  if (threadIdx.x == 0) q.group = atomicAdd(G.counter, 1u);
+  __syncthreads();
+  const uint32_t gw = q.group;
+  __syncthreads();
+  return gw;
+}
+
+// The walk's state, the same in every warp of the group.
+struct Frontier {
+  int top, nfar, nquad, nleaf;
+};
+
+enum { kActDone = 0, kActStep = 1, kActFar = 2, kActQuad = 3, kActLeaf = 4 };
+
+// Full batches first, then the walk, and what is left at its end.
+template <int W>
+__device__ __forceinline__ int coop_action(const Frontier& f) {
+  const int full = f.top > 0 ? 32 * W : 1;
+  if (f.nfar >= full) return kActFar;
+  if (f.nleaf >= full) return kActLeaf;
+  if (f.nquad >= full) return kActQuad;
+  return f.top > 0 ? kActStep : kActDone;
+}
+
+// Takes the last (at most 32 W) entries off the list of `act` and returns the
+// warp's share of them, at most 32.
+struct Share {
+  int first, cnt;
+};
+template <int W>
+__device__ __forceinline__ Share coop_share(Frontier& f, int act, int warp) {
+  int n = act == kActFar ? f.nfar : act == kActQuad ? f.nquad : f.nleaf;
+  const int take = min(n, 32 * W);
+  n -= take;
+  if (act == kActFar) f.nfar = n;
+  if (act == kActQuad) f.nquad = n;
+  if (act == kActLeaf) f.nleaf = n;
+  const int each = (take + W - 1) / W;
+  const int lo = min(warp * each, take);
+  return Share{n + lo, min(each, take - lo)};
+}
+
+// Up to 32 leaves, one per lane, read as one run of particles: lane l's leaf
+// holds the run's positions [excl, excl + count).
+struct LeafShare {
+  int start, excl, total;
+  bool valid;
+};
+
+__device__ __forceinline__ LeafShare leaf_share(const int2* leaf, int cnt, int lane) {
+  LeafShare s;
+  s.valid = lane < cnt;
+  const int2 r = s.valid ? leaf[lane] : make_int2(0, 0);
+  int inc = r.y;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += v;
+  }
+  s.start = r.x;
+  s.excl = inc - r.y;
+  s.total = __shfl_sync(0xffffffffu, inc, 31);
+  return s;
+}
+
+// The particle at the run's position b + lane, or -1 past its end. Leaves
+// hold at least one particle, so their first positions are distinct.
+__device__ __forceinline__ int leaf_particle(const LeafShare& s, int b, int lane) {
+  const int before = __popc(__ballot_sync(0xffffffffu, s.valid && s.excl < b));
+  const bool here = s.valid && s.excl >= b && s.excl < b + 32;
+  const uint32_t heads = __reduce_or_sync(0xffffffffu, here ? 1u << (s.excl - b) : 0u);
+  const int l = before + __popc(heads & (0xffffffffu >> (31 - lane))) - 1;
+  const int start = __shfl_sync(0xffffffffu, s.start, l & 31), excl = __shfl_sync(0xffffffffu, s.excl, l & 31);
+  return b + lane < s.total ? start + b + lane - excl : -1;
+}
+
+// The group's box into shared memory and its root onto the stack.
+template <int W>
+__device__ __forceinline__ void coop_begin(WalkQueues<W>& q, const float* gmin, const float* gmax, const int2& root,
+                                           int warp, int lane) {
+  if (warp == 0 && lane == 0) {
+    float c4[4];
+    lq_group_centre(gmin, gmax, c4);
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      q.box[d] = gmin[d];
+      q.box[3 + d] = gmax[d];
+    }
+#pragma unroll
+    for (int d = 0; d < 4; d++) q.box[6 + d] = c4[d];
+    q.stack[0] = root.x;
+  }
+  __syncthreads();
+}
+
+__device__ __forceinline__ Frontier coop_frontier(const int2& root) {
+  return Frontier{root.x < root.y ? 1 : 0, 0, 0, 0};
+}
+
+// The linearized quadrupole of one node (the lane's), COM A: adds a_q and J
+// about the group centre c to the lane's sums and, when node_adj is given, the
+// node's dL/dX and dL/dS (three vector reductions) from the group's cotangent
+// sums wv = (W, V).
+template <bool ADJ>
+__device__ __forceinline__ void lq_eval(const NodeRec* nd, const float4& A, const float* c, WarpShared<ADJ>& my,
+                                        float eps2, const float* wv, float* __restrict__ node_adj, int lane) {
+  const float4 Qd = __ldg(&nd->quad), X2 = __ldg(&nd->quad2);
+  const float x[3] = {c[0] - A.x, c[1] - A.y, c[2] - A.z};
+  const float S[6] = {Qd.x, Qd.y, Qd.z, Qd.w, X2.x, X2.y};
+  float a[3], J[6], f[4];
+  lq_field(x, S, eps2, a, J, f);
+#pragma unroll
+  for (int d = 0; d < 3; d++) my.acc[d][lane] += a[d];
+#pragma unroll
+  for (int d = 0; d < 6; d++) my.acc[3 + d][lane] += J[d];
+  if (ADJ && node_adj) {
+    float W[3], V[6], g[3], G[6];
+#pragma unroll
+    for (int d = 0; d < 3; d++) W[d] = wv[d];
+#pragma unroll
+    for (int d = 0; d < 6; d++) V[d] = wv[3 + d];
+    lq_node_adjoint(x, S, J, f, W, V, g, G);
+    red_add4(node_adj, -g[0], -g[1], -g[2], 0.0f);
+    red_add4(node_adj + 4, G[0], G[1], G[2], G[3]);
+    red_add2(node_adj + 8, G[4], G[5]);
+  }
+}
+
+// The walks are compiled twice: up to four targets per lane (groups of up to
+// 128) and up to two (up to 64), each for the occupancy that suits it; inside,
+// a group runs the loop of its own number of slots, so a group of 96 costs three
+// slots. Clustered systems gain from the larger groups, near-uniform ones and
+// walks bounded by a prune radius from the smaller, which the two-slot kernels
+// serve at more warps per SM. A tree walks with the kernels of its current group
+// size (sbh_native_set_group_size). Measured on a B200, 2^20 particles: force at
+// 4 blocks per SM 9.6 ms, at 5 (96 registers, spilling) 10.1; adjoint at 4 blocks
+// 23.7 ms, at 3 24.6.
 namespace tpl2 {
 constexpr int kTPL = 2;
 constexpr int kForceWalkMinBlocks = 7;
 constexpr int kAdjointWalkMinBlocks = 7;
-#define SBH_NT_WITH_WN_WALK  // the winding-number walk (groups of 32 queries) only here
 #include "sbh_native_walks.inc"
-#undef SBH_NT_WITH_WN_WALK
 }  // namespace tpl2
-
-namespace tpl3 {
-constexpr int kTPL = 3;
-constexpr int kForceWalkMinBlocks = 6;
-constexpr int kAdjointWalkMinBlocks = 5;
-#include "sbh_native_walks.inc"
-}  // namespace tpl3
 
 namespace tpl4 {
 constexpr int kTPL = 4;
-constexpr int kForceWalkMinBlocks = 5;
+constexpr int kForceWalkMinBlocks = 4;
 constexpr int kAdjointWalkMinBlocks = 4;
 #include "sbh_native_walks.inc"
 }  // namespace tpl4
@@ -943,6 +1051,13 @@ constexpr int kAdjointWalkMinBlocks = 4;
   ((QUADV)  ? NS::KERNEL<true, false, false>                                                  \
    : (PERV) ? ((CUTV) ? NS::KERNEL<false, true, true> : NS::KERNEL<false, false, true>)       \
             : ((CUTV) ? NS::KERNEL<false, true, false> : NS::KERNEL<false, false, false>))
+
+#define SBH_NT_SELECT_W(NS, KERNEL, W, QUADV, PERV, CUTV)                                       \
+  ((QUADV)  ? NS::KERNEL<W, true, false, false>                                                 \
+   : (PERV) ? ((CUTV) ? NS::KERNEL<W, false, true, true> : NS::KERNEL<W, false, false, true>)   \
+            : ((CUTV) ? NS::KERNEL<W, false, true, false> : NS::KERNEL<W, false, false, false>))
+
+#include "sbh_native_winding.inc"
 
 #include "sbh_native_stochastic.inc"
 
@@ -1155,6 +1270,7 @@ struct Layout {
   int8_t* lv;
   uint32_t* base;  // n + 1 node-slot offsets
   NodeRec* nodes;
+  int4* child;  // per node the indices of its up to eight children (-1: none)
   DVec<10>* P;
   DVec<10>* ptmp;
   DVec<3>* PN;
@@ -1212,6 +1328,7 @@ void carve(C& c, int64_t n, int nseg, int S, bool normals, bool adjoint, Layout&
   L.lv = c.template take<int8_t>(nn);
   L.base = c.template take<uint32_t>(nn + 1);
   L.nodes = c.template take<NodeRec>(cap);
+  L.child = c.template take<int4>(2 * cap);
   L.P = c.template take<DVec<10>>(nn + 1);
   L.ptmp = c.template take<DVec<10>>(scan_tiles<DVec<10>>(nn));
   L.sp = c.template take<float4>(nn);
@@ -1416,8 +1533,8 @@ int sbh_native_build(cudaStream_t stream, const float* points, const float* mass
     if (e == cudaSuccess && normals)
       e = exclusive_scan<DVec<3>>(stream, NormalMomentLoad{L.sp, L.sn}, n, L.PN, L.pntmp, true);
     if (e != cudaSuccess) return fail(SBH_ERR_CUDA, cudaGetErrorString(e));
-    finalize_nodes_kernel<<<gs(static_cast<int64_t>(L.cap)), 256, 0, stream>>>(L.nodes, L.meta, L.k0, sseg, L.boxes,
-                                                                                L.P, L.PN, L.nnrm);
+    finalize_nodes_kernel<<<gs(static_cast<int64_t>(L.cap)), 256, 0, stream>>>(L.nodes, L.child, L.meta, L.k0, sseg,
+                                                                                L.boxes, L.P, L.PN, L.nnrm);
   } else {
     e = cudaMemsetAsync(L.base, 0, sizeof(uint32_t), stream);
     if (e != cudaSuccess) return fail(SBH_ERR_CUDA, cudaGetErrorString(e));
@@ -1469,7 +1586,7 @@ __global__ void zero_node_adj_kernel(float* adj, const uint32_t* meta) {
     adj[i] = 0.0f;
 }
 
-WalkTree tree_view(const Layout& L) { return WalkTree{L.nodes, L.sp, L.sn, L.nnrm, L.roots}; }
+WalkTree tree_view(const Layout& L) { return WalkTree{L.nodes, L.child, L.sp, L.sn, L.nnrm, L.roots}; }
 
 WalkTargets self_targets(const Layout& L, const Header& h) {
   return WalkTargets{L.sp,      L.v0, L.groups, L.meta + 1, 1, L.work, static_cast<uint32_t>(h.n + h.nseg + 1),
@@ -1482,7 +1599,7 @@ bool partial_range(const Header& h) { return h.tbeg > 0 || h.tend < h.n; }
 // than one warp per possible group. Occupancy is queried per kernel and
 // device once (a host-side query; nothing is enqueued).
 template <typename K>
-unsigned walk_blocks(K kernel, int64_t max_groups) {
+unsigned walk_blocks(K kernel, int64_t max_groups, int per_block = 4, int threads = 128, size_t smem = 0) {
   struct Key {
     const void* k;
     int dev;
@@ -1502,25 +1619,60 @@ unsigned walk_blocks(K kernel, int64_t max_groups) {
   if (resident == 0) {
     int sms = 0, per_sm = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 128, 0) != cudaSuccess || per_sm <= 0)
-      per_sm = 4;
+    if (smem > 0)
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) != cudaSuccess || per_sm <= 0)
+      per_sm = 1;
     resident = static_cast<unsigned>(sms * per_sm);
     std::lock_guard<std::mutex> lk(mu);
     cache[key] = resident;
   }
-  int64_t need = (max_groups + 3) / 4;
+  int64_t need = (max_groups + per_block - 1) / per_block;
   if (need < 1) need = 1;
   return need < resident ? static_cast<unsigned>(need) : resident;
 }
 
-// Zeroes the work counter and launches a persistent walk over the groups.
-template <typename K, typename... A>
+// Zeroes the work counter and launches a persistent walk over the groups by
+// blocks of 128 threads that serve PER_BLOCK groups at a time.
+template <int PER_BLOCK = 4, typename K, typename... A>
 cudaError_t launch_walk(cudaStream_t stream, uint32_t* counter, int64_t max_groups, K kernel, A... args) {
   cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(uint32_t), stream);
   if (e != cudaSuccess) return e;
-  kernel<<<walk_blocks(kernel, max_groups), 128, 0, stream>>>(args...);
+  kernel<<<walk_blocks(kernel, max_groups, PER_BLOCK), 128, 0, stream>>>(args...);
   return cudaGetLastError();
 }
+
+// A walk by blocks of W warps, one group at a time.
+template <int W, bool ADJ, typename K, typename... A>
+cudaError_t launch_coop(cudaStream_t stream, uint32_t* counter, int64_t max_groups, K kernel, A... args) {
+  cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(uint32_t), stream);
+  if (e != cudaSuccess) return e;
+  constexpr size_t kSmem = sizeof(CoopShared<W, ADJ>);
+  const unsigned blocks = walk_blocks(kernel, max_groups, 1, 32 * W, kSmem);
+  kernel<<<blocks, 32 * W, kSmem, stream>>>(args...);
+  return cudaGetLastError();
+}
+
+#define SBH_NT_LAUNCH_W(W, ADJ, KERNEL, ...)                                                                    \
+  launch_coop<W, ADJ>(stream, L.work, h.n + h.nseg,                                                             \
+                      h.group_size > kGroupTwoSlots                                                             \
+                          ? SBH_NT_SELECT_W(tpl4, KERNEL, W, params->quadrupole, params->periodic != 0,         \
+                                            params->cutoff > 0.0f)                                              \
+                          : SBH_NT_SELECT_W(tpl2, KERNEL, W, params->quadrupole, params->periodic != 0,         \
+                                            params->cutoff > 0.0f),                                             \
+                      __VA_ARGS__)
+#define SBH_NT_LAUNCH_COOP(ADJ, KERNEL, ...)                       \
+  e = coop_wide(h) ? SBH_NT_LAUNCH_W(16, ADJ, KERNEL, __VA_ARGS__) \
+                   : SBH_NT_LAUNCH_W(4, ADJ, KERNEL, __VA_ARGS__)
+
+// Warps per group: 16 while the groups (estimated as three quarters full) are
+// fewer than 12 per SM, else 4. Force / force + adjoint in ms on a B200 with 4
+// and 16 warps: Plummer spheres of 10^4 particles (groups of 128) 0.43 / 0.91
+// and 0.14 / 0.38, 10^5 2.02 / 4.63 and 1.49 / 3.74, 2 x 10^5 2.13 / 4.81 and
+// 2.31 / 5.01, 4 x 10^5 3.77 / 9.00 and 4.26 / 9.80; a uniform cube of 10^5 in
+// groups of 64 0.53 / 1.39 and 0.72 / 1.51. Eight warps lie between the two
+// everywhere but at 10^5, where they are within 5% of the better.
+bool coop_wide(const Header& h) { return h.n * 4 / (h.group_size * 3) + h.nseg <= 12 * 148; }
 
 int check_params(const sbh_native_params* p) {
   if (!p) return invalid("params must be non-null");
@@ -1567,9 +1719,8 @@ int refresh_counts(cudaStream_t stream, const void* ws, const Header& h, const L
   WalkParams wp = walk_params(&p);
   bool cut = p.cutoff > 0.0f;
   bool per = p.periodic != 0;
-  auto k = h.group_size > kGroupThreeSlots ? SBH_NT_SELECT(tpl4, count_walk_kernel, p.quadrupole, per, cut)
-           : h.group_size > kGroupTwoSlots ? SBH_NT_SELECT(tpl3, count_walk_kernel, p.quadrupole, per, cut)
-                                           : SBH_NT_SELECT(tpl2, count_walk_kernel, p.quadrupole, per, cut);
+  auto k = h.group_size > kGroupTwoSlots ? SBH_NT_SELECT(tpl4, count_walk_kernel, p.quadrupole, per, cut)
+                                         : SBH_NT_SELECT(tpl2, count_walk_kernel, p.quadrupole, per, cut);
   e = launch_walk(stream, L.work, h.n + h.nseg, k, tree_view(L), self_targets(L, hr), wp, L.counters);
   if (e != cudaSuccess) return fail(SBH_ERR_CUDA, cudaGetErrorString(e));
   std::lock_guard<std::mutex> lk(g_reg_mu);
@@ -1638,13 +1789,7 @@ int sbh_native_force(cudaStream_t stream, const sbh_native_params* params, float
   if (partial_range(h)) e = cudaMemsetAsync(force_out, 0, h.n * 3 * sizeof(float), stream);
   if (e != cudaSuccess) return fail(SBH_ERR_CUDA, cudaGetErrorString(e));
   WalkParams wp = walk_params(params);
-  int64_t mg = h.n + h.nseg;
-  bool cut = params->cutoff > 0.0f;
-  bool per = params->periodic != 0;
-  auto k = h.group_size > kGroupThreeSlots ? SBH_NT_SELECT(tpl4, force_walk_kernel, params->quadrupole, per, cut)
-           : h.group_size > kGroupTwoSlots ? SBH_NT_SELECT(tpl3, force_walk_kernel, params->quadrupole, per, cut)
-                                           : SBH_NT_SELECT(tpl2, force_walk_kernel, params->quadrupole, per, cut);
-  e = launch_walk(stream, L.work, mg, k, tree_view(L), self_targets(L, h), wp, force_out);
+  SBH_NT_LAUNCH_COOP(false, force_walk_kernel, tree_view(L), self_targets(L, h), wp, force_out);
   if (e != cudaSuccess) return fail(SBH_ERR_CUDA, cudaGetErrorString(e));
   remember_walk(workspace, 1, params);
   return check_launch("sbh_native_force");
@@ -1669,13 +1814,8 @@ int sbh_native_adjoint_walk(cudaStream_t stream, const sbh_native_params* params
   if (e != cudaSuccess) return fail(SBH_ERR_CUDA, cudaGetErrorString(e));
   zero_node_adj_kernel<<<gs(L.cap * kNodeAdj), 256, 0, stream>>>(L.node_adj, L.meta);
   WalkParams wp = walk_params(params);
-  bool cut = params->cutoff > 0.0f;
-  bool per = params->periodic != 0;
-  auto k = h.group_size > kGroupThreeSlots ? SBH_NT_SELECT(tpl4, adjoint_walk_kernel, params->quadrupole, per, cut)
-           : h.group_size > kGroupTwoSlots ? SBH_NT_SELECT(tpl3, adjoint_walk_kernel, params->quadrupole, per, cut)
-                                           : SBH_NT_SELECT(tpl2, adjoint_walk_kernel, params->quadrupole, per, cut);
-  e = launch_walk(stream, L.work, n + h.nseg, k, tree_view(L), self_targets(L, h), wp, cotangent, force_out, L.gq,
-                  L.node_adj, L.part_adj);
+  SBH_NT_LAUNCH_COOP(true, adjoint_walk_kernel, tree_view(L), self_targets(L, h), wp, cotangent, force_out, L.gq,
+                     L.node_adj, L.part_adj);
   if (e != cudaSuccess) return fail(SBH_ERR_CUDA, cudaGetErrorString(e));
   remember_walk(workspace, 1, params);
   return check_launch("sbh_native_adjoint_walk");
@@ -1841,8 +1981,9 @@ int sbh_native_winding_number(cudaStream_t stream, float beta, const float* quer
   e = cudaMemsetAsync(L.counters, 0, kCounters * sizeof(unsigned long long), stream);
   if (e != cudaSuccess) return fail(SBH_ERR_CUDA, cudaGetErrorString(e));
   WalkTargets G{tp, qperm, groups, qmeta, 0, qmeta + 2, static_cast<uint32_t>(nq / kQueryGroup + 1), 0, INT64_MAX};
-  e = launch_walk(stream, qmeta + 2, nq / kQueryGroup + 1, tpl2::wn_walk_kernel, tree_view(L), G, beta, out,
-                  L.counters);
+  WalkParams wp{};
+  wp.beta = beta;
+  e = launch_walk<1>(stream, qmeta + 2, nq / kQueryGroup + 1, wn_walk_kernel, tree_view(L), G, wp, out, L.counters);
   if (e != cudaSuccess) return fail(SBH_ERR_CUDA, cudaGetErrorString(e));
   remember_walk(workspace, 2, nullptr);
   return check_launch("sbh_native_winding_number");
@@ -1899,8 +2040,10 @@ int sbh_native_winding_number_vjp(cudaStream_t stream, float beta, const float* 
     const uint32_t* qperm = which == 0 ? v0 : v1;
     query_gather_kernel<<<gs(nq), 256, 0, stream>>>(queries, qperm, nq, tp, groups, qmeta);
     WalkTargets G{tp, qperm, groups, qmeta, 0, qmeta + 2, static_cast<uint32_t>(nq / kQueryGroup + 1), 0, INT64_MAX};
-    e = launch_walk(stream, qmeta + 2, nq / kQueryGroup + 1, tpl2::wn_adjoint_walk_kernel, tree_view(L), G, beta,
-                    cotangent, out, grad_queries, L.node_adj, L.part_adj, L.gq);
+    WalkParams wp{};
+    wp.beta = beta;
+    e = launch_walk<1>(stream, qmeta + 2, nq / kQueryGroup + 1, wn_adjoint_walk_kernel, tree_view(L), G, wp, cotangent,
+                       out, grad_queries, L.node_adj, L.part_adj, L.gq);
     if (e != cudaSuccess) return fail(SBH_ERR_CUDA, cudaGetErrorString(e));
   }
   if (n > 0) {
