@@ -35,68 +35,10 @@
 namespace sbh {
 
 // ---------------------------------------------------------------------------
-// Direct sums (src/sbh_ffi.cu:399-546), shared-memory tiled, one query per
-// thread, Kahan-compensated across tiles.
+// Direct potential (src/sbh_ffi.cu:399-429), shared-memory tiled, one query
+// per thread, Kahan-compensated across tiles.
 // ---------------------------------------------------------------------------
 constexpr int kDirectThreads = 256;
-
-template <int VJP, bool PER>
-__global__ void __launch_bounds__(kDirectThreads)
-    direct_soft_kernel(const float* __restrict__ pts, const float* __restrict__ masses, int64_t n,
-                       const float* __restrict__ queries, const float* __restrict__ cot, int64_t nq,
-                       float* __restrict__ out, Soft s, Periodic per) {
-  __shared__ float4 tile[kDirectThreads];
-  int64_t qi = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  bool active = qi < nq;
-  float qx = 0.f, qy = 0.f, qz = 0.f, gx = 0.f, gy = 0.f, gz = 0.f;
-  if (active) {
-    qx = queries[3 * qi];
-    qy = queries[3 * qi + 1];
-    qz = queries[3 * qi + 2];
-    if (VJP) {
-      gx = cot[3 * qi];
-      gy = cot[3 * qi + 1];
-      gz = cot[3 * qi + 2];
-    }
-  }
-  float inv_l = (per.on && per.box > 0.0f) ? 1.0f / per.box : 0.0f;
-  float sx = 0.f, sy = 0.f, sz = 0.f, cx = 0.f, cy = 0.f, cz = 0.f;
-  for (int64_t base = 0; base < n; base += kDirectThreads) {
-    int64_t j = base + threadIdx.x;
-    tile[threadIdx.x] =
-        j < n ? make_float4(pts[3 * j], pts[3 * j + 1], pts[3 * j + 2], masses[j]) : make_float4(0.f, 0.f, 0.f, 0.f);
-    __syncthreads();
-    int cnt = static_cast<int>(n - base < kDirectThreads ? n - base : kDirectThreads);
-    float ax = 0.f, ay = 0.f, az = 0.f;
-#pragma unroll 4
-    for (int k = 0; k < cnt; k++) {
-      float4 p = tile[k];
-      float rx = qx - p.x, ry = qy - p.y, rz = qz - p.z;
-      if (PER) {
-        rx = min_image_rint(rx, inv_l, per);
-        ry = min_image_rint(ry, inv_l, per);
-        rz = min_image_rint(rz, inv_l, per);
-      }
-      if (VJP) {
-        soft_vjp_accum(rx, ry, rz, p.w, gx, gy, gz, s, ax, ay, az);
-      } else {
-        float c = soft_coeff(rx * rx + ry * ry + rz * rz, p.w, s);
-        ax += c * rx;
-        ay += c * ry;
-        az += c * rz;
-      }
-    }
-    kahan_add(sx, cx, ax);
-    kahan_add(sy, cy, ay);
-    kahan_add(sz, cz, az);
-    __syncthreads();
-  }
-  if (active) {
-    out[3 * qi] = sx;
-    out[3 * qi + 1] = sy;
-    out[3 * qi + 2] = sz;
-  }
-}
 
 __global__ void __launch_bounds__(kDirectThreads)
     bruteforce_gravity_kernel(const float* __restrict__ pts, const float* __restrict__ masses, int64_t n,
@@ -669,168 +611,192 @@ __device__ __forceinline__ bool o8_in_cell(float px, float py, float pz, const O
   return fabsf(px - nd.cx) <= h && fabsf(py - nd.cy) <= h && fabsf(pz - nd.cz) <= h;
 }
 
-// Direct softened sums without a periodic box, two queries per thread (q
-// and q + blockDim.x of the block's 2 blockDim.x queries). Particles are
-// staged per tile already splatted ((x, x), (y, y), (z, z), (-m, -m)), so each
-// shared-memory read lands in a packed register pair. When every pair of the
-// tile with the block's queries lies in the att = 1 range (the farthest
-// corners of the two bounding boxes, with margins, inside the unity radius:
-// always so under the "no cutoff" convention), each particle meets both
-// queries in one pass of FFMA2 / FADD2 / FMUL2 in the fixed order of
-// o8_soft_force and o8_soft_vjp, with the tile sums packed too. Otherwise the
-// tile takes those scalar forms query by query. Both round every component
-// the same way. Each tile's sum joins the query's Kahan-compensated total,
-// as in direct_soft_kernel.
-struct __align__(16) DirectSplat {
-  F2 x, y, z, nm;
+// Direct softened sums (src/sbh_ffi.cu:431-546). A block of 16 warps stages
+// tiles of 512 sources component by component, and each warp sums its 32
+// queries (one per lane) over a 1 / SPLIT share of every tile; the SPLIT warps of
+// the same queries then add their sums in order. With one query per lane the
+// packed arithmetic takes two consecutive sources per FFMA2 / FADD2 / FMUL2. A
+// chunk of 32 sources whose pairs with the warp's queries all lie in the
+// att = 1 range (the farthest corners of the two bounding boxes, with margins,
+// inside the unity radius: always so under the "no cutoff" convention) is
+// summed without a per-pair test; otherwise it takes the scalar form pair by
+// pair. Both round every component the same way (o8_soft_force, o8_soft_vjp).
+// Each tile's sum joins the query's Kahan-compensated total.
+constexpr int kDirectWarps = 16;
+constexpr int kDirectTile = 32 * kDirectWarps;
+
+struct __align__(16) DirectTile {
+  float x[kDirectTile], y[kDirectTile], z[kDirectTile], nm[kDirectTile];
+  float box[kDirectWarps][8];  // per chunk of 32: minima, maxima
 };
 
-constexpr int kDirectWarps = kDirectThreads / 32;
-
-// Box of the block's values: v[0..2] minima, v[3..5] maxima over the warp,
-// then over the warps through part[kDirectWarps][8] (the caller syncs the
-// block between the two calls).
-__device__ __forceinline__ void direct_box_warp(float* v, float (*part)[8]) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-      v[d] = fminf(v[d], __shfl_xor_sync(0xffffffffu, v[d], o));
-      v[3 + d] = fmaxf(v[3 + d], __shfl_xor_sync(0xffffffffu, v[3 + d], o));
-    }
-  if ((threadIdx.x & 31) == 0)
-    for (int d = 0; d < 6; d++) part[threadIdx.x >> 5][d] = v[d];
+__device__ __forceinline__ float warp_min(float v) {
+  float r;
+  asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+__device__ __forceinline__ float warp_max(float v) {
+  float r;
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
 }
 
-__device__ __forceinline__ void direct_box_block(float* v, const float (*part)[8]) {
-  for (int d = 0; d < 3; d++) {
-    v[d] = part[0][d];
-    v[3 + d] = part[0][3 + d];
-  }
-  for (int w = 1; w < kDirectWarps; w++)
-    for (int d = 0; d < 3; d++) {
-      v[d] = fminf(v[d], part[w][d]);
-      v[3 + d] = fmaxf(v[3 + d], part[w][3 + d]);
-    }
+template <bool PER>
+__device__ __forceinline__ float direct_image(float d, float inv_l, const Periodic& per) {
+  return PER ? min_image_rint(d, inv_l, per) : d;
+}
+template <bool PER>
+__device__ __forceinline__ F2 direct_image(F2 d, float inv_l, const Periodic& per) {
+  if (!PER) return d;
+  float a, b;
+  f2_unpack(d, a, b);
+  return f2_pack(min_image_rint(a, inv_l, per), min_image_rint(b, inv_l, per));
 }
 
-template <bool VJP>
-__global__ void __launch_bounds__(kDirectThreads, 4)
-    direct_soft2_kernel(const float* __restrict__ pts, const float* __restrict__ masses, int64_t n,
-                        const float* __restrict__ queries, const float* __restrict__ cot, int64_t nq,
-                        float* __restrict__ out, Soft s) {
-  __shared__ DirectSplat tile[kDirectThreads];
-  __shared__ float qpart[kDirectWarps][8], tpart[kDirectWarps][8];
-  const int64_t qa = static_cast<int64_t>(blockIdx.x) * (2 * kDirectThreads) + threadIdx.x;
-  const int64_t qb = qa + kDirectThreads;
-  float q[2][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}}, g[2][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
-#pragma unroll
-  for (int t = 0; t < 2; t++) {
-    const int64_t qi = t ? qb : qa;
-    if (qi < nq) {
-      for (int d = 0; d < 3; d++) {
-        q[t][d] = queries[3 * qi + d];
-        if (VJP) g[t][d] = cot[3 * qi + d];
-      }
-    }
+template <int SPLIT, bool VJP, bool PER>
+__global__ void __launch_bounds__(32 * kDirectWarps, 2)
+    direct_soft_kernel(const float* __restrict__ pts, const float* __restrict__ masses, int64_t n,
+                       const float* __restrict__ queries, const float* __restrict__ cot, int64_t nq,
+                       float* __restrict__ out, Soft s, Periodic per) {
+  __shared__ DirectTile T;
+  __shared__ float part[SPLIT > 1 ? kDirectWarps : 1][3][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int kChunks = kDirectWarps / SPLIT;  // chunks of 32 sources per warp and tile
+  const int slice = warp % SPLIT;
+  const int64_t qi = (static_cast<int64_t>(blockIdx.x) * (kDirectWarps / SPLIT) + warp / SPLIT) * 32 + lane;
+  const bool active = qi < nq;
+  const int64_t ql = active ? qi : nq - 1;
+  const float qx = queries[3 * ql], qy = queries[3 * ql + 1], qz = queries[3 * ql + 2];
+  float gx = 0.f, gy = 0.f, gz = 0.f;
+  if (VJP) {
+    gx = cot[3 * ql];
+    gy = cot[3 * ql + 1];
+    gz = cot[3 * ql + 2];
   }
-  float qbox[6];
-  for (int d = 0; d < 3; d++) {
-    qbox[d] = fminf(q[0][d], q[1][d]);
-    qbox[3 + d] = fmaxf(q[0][d], q[1][d]);
-  }
-  direct_box_warp(qbox, qpart);
-  const F2 QX = f2_pack(q[0][0], q[1][0]), QY = f2_pack(q[0][1], q[1][1]), QZ = f2_pack(q[0][2], q[1][2]);
-  const F2 GX = f2_pack(g[0][0], g[1][0]), GY = f2_pack(g[0][1], g[1][1]), GZ = f2_pack(g[0][2], g[1][2]);
+  const float qbox[6] = {warp_min(qx), warp_min(qy), warp_min(qz), warp_max(qx), warp_max(qy), warp_max(qz)};
+  const float inv_l = PER ? 1.0f / per.box : 0.0f;
+  const F2 QX = f2_pack(qx, qx), QY = f2_pack(qy, qy), QZ = f2_pack(qz, qz);
+  const F2 GX = f2_pack(gx, gx), GY = f2_pack(gy, gy), GZ = f2_pack(gz, gz);
   const float eps2 = o8_mul(s.eps, s.eps);
-  const F2 EPS2 = f2_pack(eps2, eps2), M3 = f2_pack(-3.0f, -3.0f), ZERO = f2_pack(0.0f, 0.0f);
-  float sum[2][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}}, comp[2][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
-  for (int64_t base = 0; base < n; base += kDirectThreads) {
-    const int64_t j = base + threadIdx.x;
-    float px = 0.f, py = 0.f, pz = 0.f, pm = 0.f;
-    float tbox[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
-    if (j < n) {
-      px = pts[3 * j];
-      py = pts[3 * j + 1];
-      pz = pts[3 * j + 2];
-      pm = masses[j];
-      tbox[0] = tbox[3] = px;
-      tbox[1] = tbox[4] = py;
-      tbox[2] = tbox[5] = pz;
+  const F2 EPS2 = f2_pack(eps2, eps2), M3 = f2_pack(-3.0f, -3.0f);
+  float sx = 0.f, sy = 0.f, sz = 0.f, cx = 0.f, cy = 0.f, cz = 0.f;
+  float px = 0.f, py = 0.f, pz = 0.f, pm = 0.f;  // the thread's source of the next tile
+  auto load = [&](int64_t j) {
+    const bool in = j < n;
+    px = in ? pts[3 * j] : 0.f;
+    py = in ? pts[3 * j + 1] : 0.f;
+    pz = in ? pts[3 * j + 2] : 0.f;
+    pm = in ? masses[j] : 0.f;
+  };
+  load(threadIdx.x);
+  for (int64_t base = 0; base < n; base += kDirectTile) {
+    T.x[threadIdx.x] = px;
+    T.y[threadIdx.x] = py;
+    T.z[threadIdx.x] = pz;
+    T.nm[threadIdx.x] = -pm;
+    if (s.cutoff > 0.0f) {
+      const bool in = base + threadIdx.x < n;
+      const float b[6] = {warp_min(in ? px : INFINITY),  warp_min(in ? py : INFINITY),  warp_min(in ? pz : INFINITY),
+                          warp_max(in ? px : -INFINITY), warp_max(in ? py : -INFINITY), warp_max(in ? pz : -INFINITY)};
+      if (lane == 0)
+        for (int d = 0; d < 6; d++) T.box[warp][d] = b[d];
     }
-    tile[threadIdx.x] = DirectSplat{f2_pack(px, px), f2_pack(py, py), f2_pack(pz, pz), f2_pack(-pm, -pm)};
-    direct_box_warp(tbox, tpart);
     __syncthreads();
-    // the farthest corners of the query box and the tile box (block-uniform)
-    bool unity = !(s.cutoff > 0.0f);
-    if (!unity) {
-      float qb6[6], tb6[6], R2 = 0.0f;
-      direct_box_block(qb6, qpart);
-      direct_box_block(tb6, tpart);
-      for (int d = 0; d < 3; d++) {
-        const float span = fmaxf(fabsf(qb6[3 + d] - tb6[d]), fabsf(tb6[3 + d] - qb6[d]));
-        const float mag = fmaxf(fmaxf(fabsf(qb6[d]), fabsf(qb6[3 + d])), fmaxf(fabsf(tb6[d]), fabsf(tb6[3 + d])));
-        const float m = span + 1e-6f * mag;
-        R2 += m * m;
+    load(base + kDirectTile + threadIdx.x);  // in flight during this tile's sums
+    const int left = static_cast<int>(n - base < kDirectTile ? n - base : kDirectTile);
+    uint32_t unity = 0xffffffffu;  // bit c: chunk slice * kChunks + c lies in the att = 1 range
+    if (s.cutoff > 0.0f) {
+      bool u = false;
+      if (lane < kChunks) {
+        const float* tb = T.box[slice * kChunks + lane];
+        float R2 = 0.0f;
+        for (int d = 0; d < 3; d++) {
+          const float span = fmaxf(fabsf(qbox[3 + d] - tb[d]), fabsf(tb[3 + d] - qbox[d]));
+          const float mag = fmaxf(fmaxf(fabsf(qbox[d]), fabsf(qbox[3 + d])), fmaxf(fabsf(tb[d]), fabsf(tb[3 + d])));
+          const float m = span + 1e-6f * mag;
+          R2 += m * m;
+        }
+        u = R2 * 1.0001f + 1e-12f < s.unity_r2;
       }
-      unity = R2 * 1.0001f + 1e-12f < s.unity_r2;
+      unity = __ballot_sync(0xffffffffu, u);
     }
-    const int cnt = static_cast<int>(n - base < kDirectThreads ? n - base : kDirectThreads);
-    float a[2][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
-    if (unity) {
-      F2 AX = ZERO, AY = ZERO, AZ = ZERO;
+    float ax = 0.f, ay = 0.f, az = 0.f;
+    F2 AX = f2_pack(0.f, 0.f), AY = AX, AZ = AX;
+    for (int c = 0; c < kChunks; c++) {
+      const int j0 = (slice * kChunks + c) * 32;
+      const int cnt = left - j0 < 32 ? left - j0 : 32;
+      if (cnt <= 0) break;
+      if ((unity >> c) & 1u) {  // sources past the last one carry mass zero
+#pragma unroll 2
+        for (int j = j0; j < j0 + cnt; j += 4) {
+          const ulonglong2 X = *reinterpret_cast<const ulonglong2*>(&T.x[j]);
+          const ulonglong2 Y = *reinterpret_cast<const ulonglong2*>(&T.y[j]);
+          const ulonglong2 Z = *reinterpret_cast<const ulonglong2*>(&T.z[j]);
+          const ulonglong2 M = *reinterpret_cast<const ulonglong2*>(&T.nm[j]);
+#pragma unroll
+          for (int h = 0; h < 2; h++) {
+            const F2 nm{h ? M.y : M.x};
+            const F2 rx = direct_image<PER>(o8_sub(QX, F2{h ? X.y : X.x}), inv_l, per);
+            const F2 ry = direct_image<PER>(o8_sub(QY, F2{h ? Y.y : Y.x}), inv_l, per);
+            const F2 rz = direct_image<PER>(o8_sub(QZ, F2{h ? Z.y : Z.x}), inv_l, per);
+            F2 r2, ir;
+            o8_soft_head(rx, ry, rz, EPS2, r2, ir);
+            const F2 ir3 = o8_mul(o8_mul(ir, ir), ir);
+            if (!VJP) {
+              const F2 k = o8_mul(nm, ir3);
+              AX = o8_fma(k, rx, AX);
+              AY = o8_fma(k, ry, AY);
+              AZ = o8_fma(k, rz, AZ);
+            } else {
+              const F2 ir5 = o8_mul(o8_mul(ir3, ir), ir);
+              const F2 rg = o8_fma(rz, GZ, o8_fma(ry, GY, o8_mul(rx, GX)));
+              const F2 nrad = o8_mul(rg, o8_mul(M3, ir5));
+              AX = o8_fma(nm, o8_fma(nrad, rx, o8_mul(ir3, GX)), AX);
+              AY = o8_fma(nm, o8_fma(nrad, ry, o8_mul(ir3, GY)), AY);
+              AZ = o8_fma(nm, o8_fma(nrad, rz, o8_mul(ir3, GZ)), AZ);
+            }
+          }
+        }
+      } else {
 #pragma unroll 4
-      for (int k = 0; k < cnt; k++) {
-        const DirectSplat p = tile[k];
-        const F2 rx = o8_sub(QX, p.x), ry = o8_sub(QY, p.y), rz = o8_sub(QZ, p.z);
-        F2 r2, ir;
-        o8_soft_head(rx, ry, rz, EPS2, r2, ir);
-        const F2 ir3 = o8_mul(o8_mul(ir, ir), ir);
-        if (!VJP) {
-          const F2 c = o8_mul(p.nm, ir3);
-          AX = o8_fma(c, rx, AX);
-          AY = o8_fma(c, ry, AY);
-          AZ = o8_fma(c, rz, AZ);
-        } else {
-          const F2 ir5 = o8_mul(o8_mul(ir3, ir), ir);
-          const F2 rg = o8_fma(rz, GZ, o8_fma(ry, GY, o8_mul(rx, GX)));
-          const F2 nrad = o8_mul(rg, o8_mul(M3, ir5));
-          AX = o8_fma(p.nm, o8_fma(nrad, rx, o8_mul(ir3, GX)), AX);
-          AY = o8_fma(p.nm, o8_fma(nrad, ry, o8_mul(ir3, GY)), AY);
-          AZ = o8_fma(p.nm, o8_fma(nrad, rz, o8_mul(ir3, GZ)), AZ);
-        }
-      }
-      f2_unpack(AX, a[0][0], a[1][0]);
-      f2_unpack(AY, a[0][1], a[1][1]);
-      f2_unpack(AZ, a[0][2], a[1][2]);
-    } else {
-      for (int k = 0; k < cnt; k++) {
-        const DirectSplat p = tile[k];
-        float x, y, z, nm, unused;
-        f2_unpack(p.x, x, unused);
-        f2_unpack(p.y, y, unused);
-        f2_unpack(p.z, z, unused);
-        f2_unpack(p.nm, nm, unused);
-#pragma unroll
-        for (int t = 0; t < 2; t++) {
-          const float rx = o8_sub(q[t][0], x), ry = o8_sub(q[t][1], y), rz = o8_sub(q[t][2], z);
+        for (int j = j0; j < j0 + cnt; j++) {
+          const float rx = direct_image<PER>(o8_sub(qx, T.x[j]), inv_l, per);
+          const float ry = direct_image<PER>(o8_sub(qy, T.y[j]), inv_l, per);
+          const float rz = direct_image<PER>(o8_sub(qz, T.z[j]), inv_l, per);
           if (VJP)
-            o8_soft_vjp(rx, ry, rz, nm, g[t][0], g[t][1], g[t][2], eps2, s, a[t][0], a[t][1], a[t][2]);
+            o8_soft_vjp(rx, ry, rz, T.nm[j], gx, gy, gz, eps2, s, ax, ay, az);
           else
-            o8_soft_force(rx, ry, rz, nm, eps2, s, a[t][0], a[t][1], a[t][2]);
+            o8_soft_force(rx, ry, rz, T.nm[j], eps2, s, ax, ay, az);
         }
       }
     }
-#pragma unroll
-    for (int t = 0; t < 2; t++)
-      for (int d = 0; d < 3; d++) kahan_add(sum[t][d], comp[t][d], a[t][d]);
+    float a, b;
+    f2_unpack(AX, a, b);
+    kahan_add(sx, cx, ax + (a + b));
+    f2_unpack(AY, a, b);
+    kahan_add(sy, cy, ay + (a + b));
+    f2_unpack(AZ, a, b);
+    kahan_add(sz, cz, az + (a + b));
     __syncthreads();
   }
+  if (SPLIT > 1) {
+    part[warp][0][lane] = sx;
+    part[warp][1][lane] = sy;
+    part[warp][2][lane] = sz;
+    __syncthreads();
+    if (slice == 0) {
 #pragma unroll
-  for (int t = 0; t < 2; t++) {
-    const int64_t qi = t ? qb : qa;
-    if (qi < nq)
-      for (int d = 0; d < 3; d++) out[3 * qi + d] = sum[t][d];
+      for (int w = 1; w < SPLIT; w++) {
+        sx += part[warp + w][0][lane];
+        sy += part[warp + w][1][lane];
+        sz += part[warp + w][2][lane];
+      }
+    }
+  }
+  if (active && slice == 0) {
+    out[3 * qi] = sx;
+    out[3 * qi + 1] = sy;
+    out[3 * qi + 2] = sz;
   }
 }
 
@@ -1278,6 +1244,32 @@ static unsigned grid_for(int64_t n, int threads) {
   return static_cast<unsigned>(b < 1 ? 1 : b);
 }
 
+// The smallest split that gives every SM two blocks (148 x 32 warps): 16 warps
+// per 32 queries up to 37,888 queries, 4 up to 151,552, else 1. A split costs a
+// share of the tile loads per warp (about 60 instructions per tile against 256
+// for 32 unattenuated sources and 1,600 attenuated ones at SPLIT 16). Against one
+// warp per 64 queries over every source (force / VJP, ms on a B200): 4,096 x
+// 4,096 with erfc on nearly every pair 1.46 / 1.61 -> 0.10 / 0.09, 60,000 x 60,000
+// 21.0 / 23.4 -> 12.9 / 16.0, 2^17 x 2^17 61.5 / 73.3 -> 48.2 / 60.0; without
+// attenuation 60,000 x 60,000 2.73 / 4.33 -> 2.52 / 4.19, 2^18 x 2^18 39.1 / 68.7
+// -> 36.8 / 67.1 (1.9e12 pairs/s, bound by the FMA pipe; the attenuated sums by
+// the instructions of erfcf).
+template <bool VJP, bool PER>
+static void direct_launch(cudaStream_t stream, const float* pts, const float* masses, int64_t n, const float* queries,
+                          const float* cot, int64_t nq, float* out, Soft s, Periodic per) {
+  constexpr int kThreads = 32 * kDirectWarps;
+  if (nq <= 148 * 32 * 32 / 4) {
+    direct_soft_kernel<16, VJP, PER>
+        <<<grid_for(nq, kThreads / 16), kThreads, 0, stream>>>(pts, masses, n, queries, cot, nq, out, s, per);
+  } else if (nq <= 148 * 32 * 32) {
+    direct_soft_kernel<4, VJP, PER>
+        <<<grid_for(nq, kThreads / 4), kThreads, 0, stream>>>(pts, masses, n, queries, cot, nq, out, s, per);
+  } else {
+    direct_soft_kernel<1, VJP, PER>
+        <<<grid_for(nq, kThreads), kThreads, 0, stream>>>(pts, masses, n, queries, cot, nq, out, s, per);
+  }
+}
+
 static unsigned grid_stride(int64_t n, int threads) {
   int64_t b = (n + threads - 1) / threads;
   if (b > 148 * 64) b = 148 * 64;
@@ -1459,14 +1451,12 @@ int sbh_direct_force_soft(cudaStream_t stream, const float* points, const float*
   if (!(cutoff_scale > 0.0f)) return invalid("cutoff_scale must be > 0");
   if (int rc = check_threads(threads)) return rc;
   if (nq == 0) return SBH_OK;
-  const bool per = periodic && box_length > 0.0f;
   const Soft soft{fmaxf(softening_scale, 0.0f), cutoff_scale};
-  if (per)
-    direct_soft_kernel<0, true><<<grid_for(nq, kDirectThreads), kDirectThreads, 0, stream>>>(
-        points, masses, n, queries, nullptr, nq, out, soft, Periodic{periodic, box_length});
+  if (periodic && box_length > 0.0f)
+    direct_launch<false, true>(stream, points, masses, n, queries, nullptr, nq, out, soft,
+                               Periodic{periodic, box_length});
   else
-    direct_soft2_kernel<false><<<grid_for(nq, 2 * kDirectThreads), kDirectThreads, 0, stream>>>(
-        points, masses, n, queries, nullptr, nq, out, soft);
+    direct_launch<false, false>(stream, points, masses, n, queries, nullptr, nq, out, soft, Periodic{0, 0.0f});
   return check_launch("direct_force_soft");
 }
 
@@ -1479,14 +1469,12 @@ int sbh_direct_force_soft_vjp(cudaStream_t stream, const float* points, const fl
   if (!(cutoff_scale > 0.0f)) return invalid("cutoff_scale must be > 0");
   if (int rc = check_threads(threads)) return rc;
   if (nq == 0) return SBH_OK;
-  const bool per = periodic && box_length > 0.0f;
   const Soft soft{fmaxf(softening_scale, 0.0f), cutoff_scale};
-  if (per)
-    direct_soft_kernel<1, true><<<grid_for(nq, kDirectThreads), kDirectThreads, 0, stream>>>(
-        points, masses, n, queries, cotangent, nq, out, soft, Periodic{periodic, box_length});
+  if (periodic && box_length > 0.0f)
+    direct_launch<true, true>(stream, points, masses, n, queries, cotangent, nq, out, soft,
+                              Periodic{periodic, box_length});
   else
-    direct_soft2_kernel<true><<<grid_for(nq, 2 * kDirectThreads), kDirectThreads, 0, stream>>>(
-        points, masses, n, queries, cotangent, nq, out, soft);
+    direct_launch<true, false>(stream, points, masses, n, queries, cotangent, nq, out, soft, Periodic{0, 0.0f});
   return check_launch("direct_force_soft_vjp");
 }
 
