@@ -282,7 +282,8 @@ __device__ __forceinline__ float o8_mass(const OctreeNode8* nodes, int idx) {
   return __ldg(&nodes[idx].contrib.mass);
 }
 
-__device__ __forceinline__ bool o8_far(const OctreeNode8& nd, float qx, float qy, float qz, float beta,
+template <typename Node>
+__device__ __forceinline__ bool o8_far(const Node& nd, float qx, float qy, float qz, float beta,
                                        const Periodic& per) {
   if (nd.is_leaf) return true;
   float dx = min_image_floor(qx - nd.cx, per);
@@ -298,7 +299,8 @@ __device__ __forceinline__ float axis_gap(float q, float lo, float hi) {
   return 0.0f;
 }
 
-__device__ __forceinline__ bool o8_prune(const OctreeNode8& nd, float qx, float qy, float qz,
+template <typename Node>
+__device__ __forceinline__ bool o8_prune(const Node& nd, float qx, float qy, float qz,
                                          int prune_on, float r_cut_sq, const Periodic& per) {
   if (!prune_on) return false;
   if (per.on && per.box > 0.0f) {
@@ -596,7 +598,8 @@ __device__ __forceinline__ void o8_chunk_sum(const O8Chunk& ch, int cnt, float q
 // farthest corner's squared distance stays under the unity radius, with an
 // absolute slack per axis (1e-6 of the magnitudes involved) and a relative
 // margin (1e-4) far above the rounding of the differences and of r^2.
-__device__ __forceinline__ bool o8_cell_unity(float qx, float qy, float qz, const OctreeNode8& nd, const Soft& s) {
+template <typename Node>
+__device__ __forceinline__ bool o8_cell_unity(float qx, float qy, float qz, const Node& nd, const Soft& s) {
   if (!(s.cutoff > 0.0f)) return true;
   const float h = nd.half_size;
   const float mx = fabsf(qx - nd.cx) + h + 1e-6f * (fabsf(qx) + fabsf(nd.cx) + h);
@@ -606,7 +609,8 @@ __device__ __forceinline__ bool o8_cell_unity(float qx, float qy, float qz, cons
   return R2 * 1.0001f + 1e-12f < s.unity_r2;
 }
 
-__device__ __forceinline__ bool o8_in_cell(float px, float py, float pz, const OctreeNode8& nd) {
+template <typename Node>
+__device__ __forceinline__ bool o8_in_cell(float px, float py, float pz, const Node& nd) {
   const float h = nd.half_size;
   return fabsf(px - nd.cx) <= h && fabsf(py - nd.cy) <= h && fabsf(pz - nd.cz) <= h;
 }
@@ -849,6 +853,43 @@ __device__ __forceinline__ uint32_t o8_leaf_end(uint32_t start, uint32_t end, co
   return start <= bd.num_leaves ? (end < bd.num_leaves ? end : bd.num_leaves) : start;
 }
 
+// For trees of up to kO8UnitLeaves particles a query's sum is taken in units: the root, each of its children and each of
+// their children with its whole subtree, in the order of the DFS. Every unit is
+// summed from zero and the units are added in order, so warps may share a
+// query's units without changing a bit of its row. (Larger trees keep the single
+// running sum of the reference's traversal: its rounding grows with the tree,
+// and the units' smaller one, though nearer the 64-bit sum, would leave the
+// reference's rows by 2e-5 at 2^18 particles against 2e-6 here.) Which entry starts a unit
+// follows from the stack's heights: the level-1 entries lie below h1, the
+// level-2 entries of the current level-1 node between h1 and h2.
+struct O8Units {
+  int h1 = 0, h2 = 0;
+  bool started = false;
+  // The level (0 root, 1, 2, or 3 for any deeper) of the entry popped from index i.
+  __device__ __forceinline__ int pop(int i) {
+    if (!started) {
+      started = true;
+      return 0;
+    }
+    if (i < h1) {
+      h1 = h2 = i;
+      return 1;
+    }
+    if (i < h2) {
+      h2 = i;
+      return 2;
+    }
+    return 3;
+  }
+  // After the children of a node of that level were pushed up to `top`.
+  __device__ __forceinline__ void pushed(int level, int top) {
+    if (level == 0) h1 = h2 = top;
+    if (level == 1) h2 = top;
+  }
+};
+constexpr int kO8MaxUnits = 1 + 8 + 64;
+constexpr uint32_t kO8UnitLeaves = 16384;
+
 template <int KERNEL>
 __global__ void __launch_bounds__(256)
     o8_bh_kernel(const Leaf3* __restrict__ leaf, const OctreeNode8* __restrict__ nodes,
@@ -865,11 +906,12 @@ __global__ void __launch_bounds__(256)
     gy = cot[3 * qi + 1];
     gz = cot[3 * qi + 2];
   }
-  float ax = 0.f, ay = 0.f, az = 0.f;
+  float ax = 0.f, ay = 0.f, az = 0.f, tx = 0.f, ty = 0.f, tz = 0.f;
   int stack[kO8Stack];
   int top = 0;
   stack[top++] = 0;
   bool overflow = false;
+  O8Units units;
   // A well-formed tree reaches each node from the root exactly once, so one
   // query pops at most num_nodes nodes. More pops mean that the caller's
   // child indices form a cycle: stop, flag it and keep the partial sum.
@@ -880,6 +922,11 @@ __global__ void __launch_bounds__(256)
       break;
     }
     int idx = stack[--top];
+    const int level = units.pop(top);
+    if (level < 3 && bd.num_leaves <= kO8UnitLeaves) {  // a new unit: the last one's sum joins the query's total
+      tx += ax, ty += ay, tz += az;
+      ax = ay = az = 0.f;
+    }
     if (o8_mass(nodes, idx) == 0.0f) continue;
     const OctreeNode8& nd = nodes[idx];
     if (KERNEL != O8_GRAV_GRAD && KERNEL != O8_GRAV_GRAD_VJP &&
@@ -905,12 +952,13 @@ __global__ void __launch_bounds__(256)
           }
         }
       }
+      units.pushed(level, top);
     }
   }
   if (overflow) raise_status(status, SBH_DEV_STACK_OVERFLOW);
-  out[3 * qi] = ax;
-  out[3 * qi + 1] = ay;
-  out[3 * qi + 2] = az;
+  out[3 * qi] = tx + ax;
+  out[3 * qi + 1] = ty + ay;
+  out[3 * qi + 2] = tz + az;
 }
 
 // Warp-cooperative form of o8_bh_kernel, for queries taken in Morton order
@@ -921,15 +969,20 @@ __global__ void __launch_bounds__(256)
 // some lane opens it, with that set of lanes. A lane's nodes thus come off
 // the stack in the order of its own per-thread DFS, so it adds the same terms
 // in the same order and every output row equals o8_bh_kernel's bit for bit;
-// node records are read once per warp instead of once per thread. At a leaf
+// node records are read once per warp instead of once per thread. The next
+// entry's record loads while the current node's terms are summed. At a leaf
 // the warp copies the particles in chunks of 32 (one coalesced load per lane)
 // into a per-warp buffer in shared memory, and the summing lanes read them
 // from there in the leaf's order.
-// The block holds blockDim.x / 32 warps (the caller's `threads`, the
-// reference's launch parameter, in whole warps). Its dynamic shared memory
-// holds each warp's leaf buffer (32 x 16 B), then each warp's stack of STACK
-// entries: 64 for a dense octree8 of depth <= 9 (a DFS of depth d holds at
-// most 7 d + 1 entries), otherwise the reference's 128.
+//
+// WQ = 8: the block's eight warps share one set of 32 queries. Every warp walks
+// the tree's top two levels and takes units (O8Units) off a counter; the units'
+// sums meet in shared memory and are added in order. WQ = 1: each warp of the
+// block has its own queries.
+// The block's dynamic shared memory holds each warp's leaf buffer (32 x 16 B),
+// then each warp's stack of STACK entries (64 for a dense octree8 of depth <= 9:
+// a DFS of depth d holds at most 7 d + 1 entries; otherwise the reference's
+// 128), then for WQ = 8 the units' sums.
 struct O8StackEntry {
   int node;
   uint32_t lanes;
@@ -939,8 +992,46 @@ __host__ __device__ constexpr size_t o8_warp_smem(int warps, int stack) {
   return static_cast<size_t>(warps) * (sizeof(O8Chunk) + stack * sizeof(O8StackEntry));
 }
 
-template <int KERNEL, int STACK, bool STAGED>
-__global__ void __launch_bounds__(1024)
+// What a visit reads of a node record.
+struct O8Visit {
+  float mass, cx, cy, cz, half_size, diameter, px, py, pz;
+  uint32_t start, end;
+  uint8_t child_mask, is_leaf;
+};
+
+__device__ __forceinline__ O8Visit o8_visit(const OctreeNode8* __restrict__ nodes, int idx) {
+  const char* p = reinterpret_cast<const char*>(nodes + idx);
+  const uint2 range = __ldg(reinterpret_cast<const uint2*>(p));
+  const uint2 fl = __ldg(reinterpret_cast<const uint2*>(p + 48));
+  const float2 yz = __ldg(reinterpret_cast<const float2*>(p + 56)), hd = __ldg(reinterpret_cast<const float2*>(p + 64));
+  const float2 xy = __ldg(reinterpret_cast<const float2*>(p + 72));
+  O8Visit v;
+  v.start = range.x;
+  v.end = range.y;
+  v.child_mask = static_cast<uint8_t>(fl.x);
+  v.is_leaf = static_cast<uint8_t>(fl.x >> 16);
+  v.cx = __uint_as_float(fl.y);
+  v.cy = yz.x;
+  v.cz = yz.y;
+  v.half_size = hd.x;
+  v.diameter = hd.y;
+  v.px = xy.x;
+  v.py = xy.y;
+  v.pz = __ldg(reinterpret_cast<const float*>(p + 80));
+  v.mass = __ldg(reinterpret_cast<const float*>(p + 96));
+  return v;
+}
+static_assert(offsetof(OctreeNode8, child_mask) == 48 && offsetof(OctreeNode8, is_leaf) == 50 &&
+                  offsetof(OctreeNode8, cx) == 52 && offsetof(OctreeNode8, half_size) == 64,
+              "OctreeNode8 offsets read by o8_visit");
+
+struct O8UnitSums {
+  float v[kO8MaxUnits][3][32];
+  int next;
+};
+
+template <int KERNEL, int STACK, bool STAGED, int WQ>
+__global__ void __launch_bounds__(256, 3)
     o8_bh_warp_kernel(const Leaf3* __restrict__ leaf, const OctreeNode8* __restrict__ nodes,
                       const float* __restrict__ queries, const float* __restrict__ cot, int64_t nq, float beta,
                       Soft s, int prune_on, float r_cut_sq, Periodic per, float* __restrict__ out, uint32_t* status,
@@ -950,10 +1041,21 @@ __global__ void __launch_bounds__(1024)
   O8Chunk& chunk = reinterpret_cast<O8Chunk*>(o8_smem)[warp];
   O8StackEntry* stack = reinterpret_cast<O8StackEntry*>(reinterpret_cast<O8Chunk*>(o8_smem) + (blockDim.x >> 5)) +
                         warp * STACK;
-  const int64_t ti = (static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + warp) * 32 + lane;
+  O8UnitSums& sums = *reinterpret_cast<O8UnitSums*>(reinterpret_cast<char*>(o8_smem) +
+                                                    o8_warp_smem(static_cast<int>(blockDim.x >> 5), STACK));
+  const int64_t set = WQ > 1 ? static_cast<int64_t>(blockIdx.x)
+                             : static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + warp;
+  const int64_t ti = set * 32 + lane;
   const bool valid = ti < nq;
   const uint32_t live = __ballot_sync(0xffffffffu, valid);
-  if (live == 0) return;  // warp-uniform
+  if (live == 0) return;  // uniform over the warps of a set
+  int mine = 0;           // WQ > 1: the unit this warp takes next
+  if (WQ > 1) {
+    if (threadIdx.x == 0) sums.next = WQ;
+    for (int i = threadIdx.x; i < kO8MaxUnits * 96; i += 32 * WQ) (&sums.v[0][0][0])[i] = 0.0f;
+    mine = warp;
+    __syncthreads();
+  }
   const int64_t qi = valid ? static_cast<int64_t>(order[ti]) : 0;
   float qx = 0.f, qy = 0.f, qz = 0.f, gx = 0.f, gy = 0.f, gz = 0.f;
   if (valid) {
@@ -966,101 +1068,141 @@ __global__ void __launch_bounds__(1024)
       gz = cot[3 * qi + 2];
     }
   }
-  float ax = 0.f, ay = 0.f, az = 0.f;
+  float ax = 0.f, ay = 0.f, az = 0.f, tx = 0.f, ty = 0.f, tz = 0.f;
+  const bool in_units = bd.num_leaves <= kO8UnitLeaves;
+  int unit = -1;  // units begun so far, less one
+  auto end_unit = [&] {  // the current unit's sum joins the total
+    if (WQ == 1) {
+      if (!in_units) return;
+      tx += ax, ty += ay, tz += az;
+    } else if (unit == mine) {
+      sums.v[unit][0][lane] = ax;
+      sums.v[unit][1][lane] = ay;
+      sums.v[unit][2][lane] = az;
+      if (lane == 0) mine = atomicAdd(&sums.next, 1);
+      mine = __shfl_sync(0xffffffffu, mine, 0);
+    }
+    ax = ay = az = 0.f;
+  };
   if (lane == 0) stack[0] = O8StackEntry{0, live};
   __syncwarp();
   int top = 1;  // warp-uniform
   bool overflow = false;
   uint32_t visits = 0;  // bounded as in o8_bh_kernel
+  O8Units units;
+  O8StackEntry en{0, live};
+  O8Visit nx = o8_visit(nodes, 0);
   while (top > 0) {
     if (++visits > bd.num_nodes) {
       if (lane == 0) raise_status(status, SBH_DEV_ITER_LIMIT);
       break;
     }
-    const O8StackEntry en = stack[--top];
-    __syncwarp();  // every lane has read the entry before it is overwritten
+    const O8Visit nd = nx;
     const int idx = en.node;
-    if (o8_mass(nodes, idx) == 0.0f) continue;
-    const OctreeNode8& nd = nodes[idx];
-    bool act = (en.lanes >> lane) & 1u;
+    const uint32_t lanes = en.lanes;
+    top--;
+    const int level = units.pop(top);
+    if (level < 3) {
+      end_unit();
+      unit++;
+    }
+    const bool own = WQ == 1 || unit == mine;
+    bool act = ((lanes >> lane) & 1u) && nd.mass != 0.0f && (own || level < 2);
     if (KERNEL != O8_GRAV_GRAD && KERNEL != O8_GRAV_GRAD_VJP)
       act = act && !o8_prune(nd, qx, qy, qz, prune_on, r_cut_sq, per);
     const bool far = act && o8_far(nd, qx, qy, qz, beta, per);
+    const uint32_t open = __ballot_sync(0xffffffffu, act && !far);
+    if (open) {
+      // slot c's child index in lane c; the pushes keep the slots' order
+      const uint32_t ch = lane < 8 ? __ldg(&nodes[idx].child[lane]) : 0u;
+      bool push = lane < 8 && ((nd.child_mask >> lane) & 1u);
+      if (push && !o8_node_ok(ch, bd, status)) push = false;
+      const uint32_t pm = __ballot_sync(0xffffffffu, push);
+      const int at = top + __popc(pm & ((1u << lane) - 1u));
+      if (push && at < STACK) stack[at] = O8StackEntry{static_cast<int>(ch), open};
+      top += __popc(pm);
+      if (top > STACK) {
+        top = STACK;
+        overflow = true;
+      }
+      units.pushed(level, top);
+    }
+    __syncwarp();
+    if (top > 0) {
+      en = stack[top - 1];
+      nx = o8_visit(nodes, en.node);
+    }
+    if (!own || !__any_sync(0xffffffffu, far)) {
+      __syncwarp();  // every lane has read the entry before it is overwritten
+      continue;
+    }
     if (nd.is_leaf && !STAGED) {  // nd is warp-uniform: every lane reads the same node
       if (far)
         o8_leaf_sum<KERNEL>(leaf, nd.start, o8_leaf_end(nd.start, nd.end, bd, status), qx, qy, qz, gx, gy, gz, s,
                             per, ax, ay, az);
     } else if (nd.is_leaf) {
-      if (__ballot_sync(0xffffffffu, far)) {
-        const uint32_t start = nd.start, end = o8_leaf_end(start, nd.end, bd, status);
-        constexpr bool kSoft = KERNEL == O8_SOFT || KERNEL == O8_SOFT_VJP;
-        const bool q_unity = !far || o8_cell_unity(qx, qy, qz, nd, s);
-        // chunks of 32 particles, one per lane, the next one loaded while
-        // the current one is summed
-        float4 nxt = make_float4(0.f, 0.f, 0.f, 0.f);
-        float nxt_m = 0.f;
-        if (start + lane < end) {
-          nxt = __ldg(reinterpret_cast<const float4*>(leaf + start + lane));
-          nxt_m = __ldg(&leaf[start + lane].mass);
+      const uint32_t start = nd.start, end = o8_leaf_end(start, nd.end, bd, status);
+      constexpr bool kSoft = KERNEL == O8_SOFT || KERNEL == O8_SOFT_VJP;
+      const bool q_unity = !far || o8_cell_unity(qx, qy, qz, nd, s);
+      // chunks of 32 particles, one per lane, the next one loaded while
+      // the current one is summed
+      float4 nxt = make_float4(0.f, 0.f, 0.f, 0.f);
+      float nxt_m = 0.f;
+      if (start + lane < end) {
+        nxt = __ldg(reinterpret_cast<const float4*>(leaf + start + lane));
+        nxt_m = __ldg(&leaf[start + lane].mass);
+      }
+      for (uint32_t c = start; c < end; c += kO8LeafChunk) {
+        const uint32_t i = c + lane;
+        bool in_cell = true;
+        if (i < end) {
+          chunk.x[lane] = nxt.x;
+          chunk.y[lane] = nxt.y;
+          chunk.z[lane] = nxt.z;
+          chunk.nm[lane] = -nxt_m;
+          in_cell = o8_in_cell(nxt.x, nxt.y, nxt.z, nd);
         }
-        for (uint32_t c = start; c < end; c += kO8LeafChunk) {
-          const uint32_t i = c + lane;
-          bool in_cell = true;
-          if (i < end) {
-            chunk.x[lane] = nxt.x;
-            chunk.y[lane] = nxt.y;
-            chunk.z[lane] = nxt.z;
-            chunk.nm[lane] = -nxt_m;
-            in_cell = o8_in_cell(nxt.x, nxt.y, nxt.z, nd);
-          }
-          if (i + kO8LeafChunk < end) {
-            nxt = __ldg(reinterpret_cast<const float4*>(leaf + i + kO8LeafChunk));
-            nxt_m = __ldg(&leaf[i + kO8LeafChunk].mass);
-          }
-          const bool unity = __all_sync(0xffffffffu, in_cell && q_unity);
-          __syncwarp();
-          const int cnt = end - c < kO8LeafChunk ? static_cast<int>(end - c) : kO8LeafChunk;
-          if (far) {
-            if (kSoft && !per.on) {
-              if (unity)
-                o8_chunk_sum<KERNEL, false>(chunk, cnt, qx, qy, qz, gx, gy, gz, s, ax, ay, az);
-              else
-                o8_chunk_sum<KERNEL, true>(chunk, cnt, qx, qy, qz, gx, gy, gz, s, ax, ay, az);
-            } else {
-              for (int j = 0; j < cnt; j++)
-                o8_pair<KERNEL>(qx, qy, qz, chunk.x[j], chunk.y[j], chunk.z[j], -chunk.nm[j], gx, gy, gz, s, per,
-                                ax, ay, az);
-            }
-          }
-          __syncwarp();  // the chunk is read before the next one overwrites it
+        if (i + kO8LeafChunk < end) {
+          nxt = __ldg(reinterpret_cast<const float4*>(leaf + i + kO8LeafChunk));
+          nxt_m = __ldg(&leaf[i + kO8LeafChunk].mass);
         }
+        const bool unity = __all_sync(0xffffffffu, in_cell && q_unity);
+        __syncwarp();
+        const int cnt = end - c < kO8LeafChunk ? static_cast<int>(end - c) : kO8LeafChunk;
+        if (far) {
+          if (kSoft && !per.on) {
+            if (unity)
+              o8_chunk_sum<KERNEL, false>(chunk, cnt, qx, qy, qz, gx, gy, gz, s, ax, ay, az);
+            else
+              o8_chunk_sum<KERNEL, true>(chunk, cnt, qx, qy, qz, gx, gy, gz, s, ax, ay, az);
+          } else {
+            for (int j = 0; j < cnt; j++)
+              o8_pair<KERNEL>(qx, qy, qz, chunk.x[j], chunk.y[j], chunk.z[j], -chunk.nm[j], gx, gy, gz, s, per, ax,
+                              ay, az);
+          }
+        }
+        __syncwarp();  // the chunk is read before the next one overwrites it
       }
     } else if (far) {
-      o8_pair<KERNEL>(qx, qy, qz, nd.contrib.pos[0], nd.contrib.pos[1], nd.contrib.pos[2], nd.contrib.mass, gx, gy,
-                      gz, s, per, ax, ay, az);
+      o8_pair<KERNEL>(qx, qy, qz, nd.px, nd.py, nd.pz, nd.mass, gx, gy, gz, s, per, ax, ay, az);
     }
-    const uint32_t open = __ballot_sync(0xffffffffu, act && !far);
-    if (open) {
-      const uint8_t mask = nd.child_mask;
-      for (int c = 0; c < 8; c++) {
-        if (mask & (1u << c)) {
-          if (!o8_node_ok(nd.child[c], bd, status)) continue;
-          if (top < STACK) {
-            if (lane == 0) stack[top] = O8StackEntry{static_cast<int>(nd.child[c]), open};
-            top++;
-          } else {
-            overflow = true;
-          }
-        }
-      }
-      __syncwarp();
-    }
+    __syncwarp();
   }
   if (overflow && lane == 0) raise_status(status, SBH_DEV_STACK_OVERFLOW);
-  if (valid) {
-    out[3 * qi] = ax;
-    out[3 * qi + 1] = ay;
-    out[3 * qi + 2] = az;
+  if (WQ == 1) {
+    if (valid) {
+      out[3 * qi] = tx + ax;
+      out[3 * qi + 1] = ty + ay;
+      out[3 * qi + 2] = tz + az;
+    }
+  } else {
+    end_unit();
+    __syncthreads();
+    for (int c = warp; c < 3; c += WQ) {
+      float t = 0.f;
+      for (int u = 0; u < kO8MaxUnits; u++) t += sums.v[u][c][lane];
+      if (valid) out[3 * qi + c] = t;
+    }
   }
 }
 
@@ -1088,13 +1230,114 @@ __device__ __forceinline__ uint32_t o8_child_slot(const OctreeNode8& nd, float p
   return ix | (iy << 1) | (iz << 2);
 }
 
+// The subdomains of the estimator (the reference's DFS from the root down to
+// leaves and nodes of depth 3) do not depend on the query, so a block lists them
+// once in shared memory, level by level: every round replaces each node that
+// is neither by its children, slot 7 first, which keeps the order of a DFS that
+// pops the last child pushed. Per thread this search was a chain of some 600
+// dependent visits and 2.5 KB of local memory. A well-formed tree ends after
+// three rounds with at most 512 entries; more nodes seen than the buffer has
+// (a cycle in the caller's child indices) or a longer list sets the status bits
+// of the per-thread search.
+constexpr int kStochThreads = 128;
+
+struct O8Subdomains {
+  uint32_t list[2][kMaxSubdomains];
+  int warp_sum[kStochThreads / 32];
+  int cur;
+};
+
+__device__ __forceinline__ int o8_subdomains(const OctreeNode8* __restrict__ nodes, const O8Bounds& bd,
+                                             uint32_t* status, O8Subdomains& S) {
+  constexpr int kPer = kMaxSubdomains / kStochThreads;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) S.list[0][0] = 0;
+  __syncthreads();
+  int n = 1, cur = 0;
+  for (uint64_t seen = 1;;) {
+    int cnt[kPer], sum = 0;
+    uint32_t id[kPer];
+    uint8_t mask[kPer];  // children that replace the entry; 0 with cnt 1: the entry itself
+    bool open = false;  // a later round is needed
+#pragma unroll
+    for (int e = 0; e < kPer; e++) {
+      const int i = static_cast<int>(threadIdx.x) * kPer + e;
+      cnt[e] = 0;
+      mask[e] = 0;
+      if (i < n) {
+        id[e] = S.list[cur][i];
+        const OctreeNode8& nd = nodes[id[e]];
+        if (nd.contrib.mass != 0.0f) {
+          if (nd.is_leaf || nd.depth >= kControlDepth) {
+            cnt[e] = 1;
+          } else {
+            for (int c = 0; c < 8; c++)
+              if (((nd.child_mask >> c) & 1u) && o8_node_ok(nd.child[c], bd, status))
+                mask[e] |= static_cast<uint8_t>(1u << c);
+            cnt[e] = __popc(mask[e]);
+            open = true;
+          }
+        }
+      }
+      sum += cnt[e] + (mask[e] ? cnt[e] << 16 : 0);  // entries; above, the new ones
+    }
+    int inc = sum;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += v;
+    }
+    if (lane == 31) S.warp_sum[warp] = inc;
+    open = __syncthreads_or(open);
+    int at = inc - sum, total = 0;
+    for (int w = 0; w < kStochThreads / 32; w++) {
+      if (w < warp) at += S.warp_sum[w];
+      total += S.warp_sum[w];
+    }
+    seen += static_cast<uint64_t>(total >> 16);
+    at &= 0xFFFF;
+    total &= 0xFFFF;
+#pragma unroll
+    for (int e = 0; e < kPer; e++) {
+      if (cnt[e] == 0) continue;
+      if (mask[e] == 0) {
+        if (at < kMaxSubdomains) S.list[cur ^ 1][at] = id[e];
+        at++;
+      } else {
+        for (int c = 7; c >= 0; c--) {
+          if (!((mask[e] >> c) & 1u)) continue;
+          if (at < kMaxSubdomains) S.list[cur ^ 1][at] = nodes[id[e]].child[c];
+          at++;
+        }
+      }
+    }
+    if (total > kMaxSubdomains) {
+      if (threadIdx.x == 0) raise_status(status, SBH_DEV_STACK_OVERFLOW);
+      total = kMaxSubdomains;
+    }
+    cur ^= 1;
+    n = total;
+    __syncthreads();
+    if (!open || n == 0) break;
+    if (seen > bd.num_nodes) {
+      if (threadIdx.x == 0) raise_status(status, SBH_DEV_ITER_LIMIT);
+      break;
+    }
+  }
+  if (threadIdx.x == 0) S.cur = cur;
+  __syncthreads();
+  return n;
+}
+
 template <int KERNEL, bool SOFTENED>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kStochThreads)
     o8_stochastic_kernel(const Leaf3* __restrict__ leaf, const OctreeNode8* __restrict__ nodes,
                          const float* __restrict__ queries, const float* __restrict__ cot, int64_t nq,
                          int samples, int seed, float beta, Soft s, int prune_on, float r_cut_sq,
                          Periodic per, float* __restrict__ out, uint32_t* status, O8Bounds bd,
                          const uint32_t* __restrict__ order) {
+  __shared__ O8Subdomains S;
+  const int nsub = o8_subdomains(nodes, bd, status, S);
+  const uint32_t* subs = S.list[S.cur];
   int64_t ti = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (ti >= nq) return;
   const int64_t qi = order ? static_cast<int64_t>(order[ti]) : ti;
@@ -1113,36 +1356,6 @@ __global__ void __launch_bounds__(256)
   curand_init(static_cast<unsigned long long>(static_cast<unsigned>(sq) + 0x9e3779b9u), 0, 0, &st2);
 
   float tx = 0.f, ty = 0.f, tz = 0.f;
-  int stack[kO8Stack];
-  int top = 0;
-  stack[top++] = 0;
-  uint32_t subs[kMaxSubdomains];
-  int nsub = 0;
-  bool overflow = false;
-  uint32_t visits = 0;  // bounded as in o8_bh_kernel
-  while (top > 0) {
-    if (++visits > bd.num_nodes) {
-      raise_status(status, SBH_DEV_ITER_LIMIT);
-      break;
-    }
-    int idx = stack[--top];
-    const OctreeNode8& nd = nodes[idx];
-    if (nd.contrib.mass == 0.0f) continue;
-    if (nd.is_leaf || nd.depth >= kControlDepth) {
-      if (nsub < kMaxSubdomains) subs[nsub++] = static_cast<uint32_t>(idx);
-      continue;
-    }
-    uint8_t mask = nd.child_mask;
-    for (int c = 0; c < 8; c++) {
-      if (mask & (1u << c)) {
-        if (!o8_node_ok(nd.child[c], bd, status)) continue;
-        if (top < kO8Stack)
-          stack[top++] = static_cast<int>(nd.child[c]);
-        else
-          overflow = true;
-      }
-    }
-  }
   for (int sd = 0; sd < nsub; sd++) {
     const OctreeNode8& sub = nodes[subs[sd]];
     if (SOFTENED && o8_prune(sub, qx, qy, qz, prune_on, r_cut_sq, per)) continue;
@@ -1225,7 +1438,6 @@ __global__ void __launch_bounds__(256)
       tz += sz / inv;
     }
   }
-  if (overflow) raise_status(status, SBH_DEV_STACK_OVERFLOW);
   out[3 * qi] = tx;
   out[3 * qi + 1] = ty;
   out[3 * qi + 2] = tz;
@@ -1323,7 +1535,7 @@ using namespace sbh;
 // code of their position in the root cell, so a warp's threads walk nearby
 // paths and the per-thread traversal diverges far less than for queries in
 // random order.
-constexpr int64_t kOrderMinQueries = 4096;
+constexpr int64_t kOrderMinQueries = 64;
 
 template <typename C>
 static void order_carve(C& c, int64_t nq, uint32_t** k0, uint32_t** v0, uint32_t** k1, uint32_t** v1,
@@ -1391,40 +1603,63 @@ static bool o8_small_stack(uint32_t num_nodes) {
 // gains little from staged particles, so that kernel sums each leaf per lane
 // straight from global memory and holds fewer registers (TreePM short range,
 // 2^21 particles: 16.6 ms against 17.7 ms staged).
-template <int KERNEL, int STACK>
-static void o8_launch_warp_kind(unsigned grid, unsigned block, size_t smem, cudaStream_t stream, const Leaf3* L,
-                                const OctreeNode8* N, const float* queries, const float* cot, int64_t nq, float beta,
-                                Soft s, int prune_on, float r_cut_sq, Periodic per, float* out, uint32_t* status,
-                                O8Bounds bd, const uint32_t* order) {
+template <int KERNEL, int STACK, int WQ>
+static void o8_launch_warp_kind(int warps, cudaStream_t stream, const Leaf3* L, const OctreeNode8* N,
+                                const float* queries, const float* cot, int64_t nq, float beta, Soft s, int prune_on,
+                                float r_cut_sq, Periodic per, float* out, uint32_t* status, O8Bounds bd,
+                                const uint32_t* order) {
+  const unsigned block = 32u * static_cast<unsigned>(warps);
+  const unsigned grid = grid_for(nq, WQ > 1 ? 32 : static_cast<int>(block));
+  const size_t smem = o8_warp_smem(warps, STACK) + (WQ > 1 ? sizeof(O8UnitSums) : 0);
   if (per.on)
-    o8_bh_warp_kernel<KERNEL, STACK, false><<<grid, block, smem, stream>>>(L, N, queries, cot, nq, beta, s, prune_on,
-                                                                           r_cut_sq, per, out, status, bd, order);
+    o8_bh_warp_kernel<KERNEL, STACK, false, WQ><<<grid, block, smem, stream>>>(
+        L, N, queries, cot, nq, beta, s, prune_on, r_cut_sq, per, out, status, bd, order);
   else
-    o8_bh_warp_kernel<KERNEL, STACK, true><<<grid, block, smem, stream>>>(L, N, queries, cot, nq, beta, s, prune_on,
-                                                                          r_cut_sq, per, out, status, bd, order);
+    o8_bh_warp_kernel<KERNEL, STACK, true, WQ><<<grid, block, smem, stream>>>(
+        L, N, queries, cot, nq, beta, s, prune_on, r_cut_sq, per, out, status, bd, order);
+}
+
+// Eight warps share 32 queries while the query sets alone give the SMs fewer
+// than 16 warps each (75,776 queries) and the sums are taken in units; else each
+// warp has its own queries and the caller's `threads` gives the warps per block
+// (at most 8: the result does not depend on it). Softened force / VJP of the
+// particles themselves, ms on a B200, shared against own: 5,000 particles 0.55 /
+// 0.56 and 2.5 / 2.6 (3.1 / 3.1 before the next node's prefetch), 20,000 1.6 / 1.6
+// and 4.2 / 4.3, 60,000 in a uniform cube 5.6 / 5.8 and 6.7 / 6.9, in a Plummer
+// sphere 7.2 / 7.5 and 6.3 / 6.8; 10^5 12.5 / 13.2 and 8.5 / 9.7 (9.6 / 10.7 before).
+static bool o8_shared_sets(int64_t nq, uint32_t leaves) { return nq <= 148 * 16 * 32 && leaves <= kO8UnitLeaves; }
+
+template <int KERNEL, int STACK, typename... A>
+static void o8_launch_warp_sets(int threads, int64_t nq, uint32_t leaves, cudaStream_t stream, A... args) {
+  if (o8_shared_sets(nq, leaves)) {
+    o8_launch_warp_kind<KERNEL, STACK, 8>(8, stream, args...);
+  } else {
+    const int warps = threads >= 64 ? (threads < 256 ? threads / 32 : 8) : 1;
+    o8_launch_warp_kind<KERNEL, STACK, 1>(warps, stream, args...);
+  }
 }
 
 template <int STACK>
-static void o8_launch_warp(int kernel, unsigned grid, unsigned block, size_t smem, cudaStream_t stream,
-                           const Leaf3* L, const OctreeNode8* N, const float* queries, const float* cot, int64_t nq,
-                           float beta, Soft s, int prune_on, float r_cut_sq, Periodic per, float* out,
-                           uint32_t* status, O8Bounds bd, const uint32_t* order) {
+static void o8_launch_warp(int kernel, int threads, cudaStream_t stream, const Leaf3* L, const OctreeNode8* N,
+                           const float* queries, const float* cot, int64_t nq, float beta, Soft s, int prune_on,
+                           float r_cut_sq, Periodic per, float* out, uint32_t* status, O8Bounds bd,
+                           const uint32_t* order) {
   switch (kernel) {
     case O8_GRAV_GRAD:
-      o8_launch_warp_kind<O8_GRAV_GRAD, STACK>(grid, block, smem, stream, L, N, queries, cot, nq, beta, s, 0, 0.f, per,
-                                               out, status, bd, order);
+      o8_launch_warp_sets<O8_GRAV_GRAD, STACK>(threads, nq, bd.num_leaves, stream, L, N, queries, cot, nq, beta, s, 0, 0.f, per, out,
+                                               status, bd, order);
       break;
     case O8_SOFT:
-      o8_launch_warp_kind<O8_SOFT, STACK>(grid, block, smem, stream, L, N, queries, cot, nq, beta, s, prune_on,
-                                          r_cut_sq, per, out, status, bd, order);
+      o8_launch_warp_sets<O8_SOFT, STACK>(threads, nq, bd.num_leaves, stream, L, N, queries, cot, nq, beta, s, prune_on, r_cut_sq,
+                                          per, out, status, bd, order);
       break;
     case O8_GRAV_GRAD_VJP:
-      o8_launch_warp_kind<O8_GRAV_GRAD_VJP, STACK>(grid, block, smem, stream, L, N, queries, cot, nq, beta, s, 0, 0.f,
-                                                   per, out, status, bd, order);
+      o8_launch_warp_sets<O8_GRAV_GRAD_VJP, STACK>(threads, nq, bd.num_leaves, stream, L, N, queries, cot, nq, beta, s, 0, 0.f, per,
+                                                   out, status, bd, order);
       break;
     default:
-      o8_launch_warp_kind<O8_SOFT_VJP, STACK>(grid, block, smem, stream, L, N, queries, cot, nq, beta, s, prune_on,
-                                              r_cut_sq, per, out, status, bd, order);
+      o8_launch_warp_sets<O8_SOFT_VJP, STACK>(threads, nq, bd.num_leaves, stream, L, N, queries, cot, nq, beta, s, prune_on, r_cut_sq,
+                                              per, out, status, bd, order);
       break;
   }
 }
@@ -1552,19 +1787,13 @@ static int o8_launch_bh(int kernel, cudaStream_t stream, const void* leaf, size_
   int orc = SBH_OK;
   const uint32_t* order = o8_query_order(stream, N, queries, nq, workspace, workspace_bytes, &orc);
   if (orc != SBH_OK) return orc;
-  if (order) {  // Morton-ordered queries: one warp walks 32 neighbours together
-    const int warps = threads >= 64 ? (threads < 1024 ? threads / 32 : 32) : 1;
-    const unsigned tw = 32u * static_cast<unsigned>(warps);
-    const unsigned gw = grid_for(nq, static_cast<int>(tw));
-    if (o8_small_stack(bd.num_nodes)) {
-      const size_t sm = o8_warp_smem(warps, 64);
-      o8_launch_warp<64>(kernel, gw, tw, sm, stream, L, N, queries, cot, nq, beta, s, prune_on, r_cut_sq, per, out,
-                         status, bd, order);
-    } else {
-      const size_t sm = o8_warp_smem(warps, kO8Stack);
-      o8_launch_warp<kO8Stack>(kernel, gw, tw, sm, stream, L, N, queries, cot, nq, beta, s, prune_on, r_cut_sq, per,
-                               out, status, bd, order);
-    }
+  if (order) {  // Morton-ordered queries: a warp walks 32 neighbours together
+    if (o8_small_stack(bd.num_nodes))
+      o8_launch_warp<64>(kernel, threads, stream, L, N, queries, cot, nq, beta, s, prune_on, r_cut_sq, per, out, status,
+                         bd, order);
+    else
+      o8_launch_warp<kO8Stack>(kernel, threads, stream, L, N, queries, cot, nq, beta, s, prune_on, r_cut_sq, per, out,
+                               status, bd, order);
     return check_launch("barnes_hut_force_octree8");
   }
   unsigned g = grid_for(nq, 256);
@@ -1675,20 +1904,20 @@ static int o8_launch_stochastic(bool vjp, int softened, cudaStream_t stream, con
   int orc = SBH_OK;
   const uint32_t* order = o8_query_order(stream, N, queries, nq, workspace, workspace_bytes, &orc);
   if (orc != SBH_OK) return orc;
-  unsigned g = grid_for(nq, 128);
+  unsigned g = grid_for(nq, kStochThreads);
   if (!vjp) {
     if (softened)
-      o8_stochastic_kernel<O8_SOFT, true><<<g, 128, 0, stream>>>(L, N, queries, cot, nq, samples, seed, beta, s, on,
+      o8_stochastic_kernel<O8_SOFT, true><<<g, kStochThreads, 0, stream>>>(L, N, queries, cot, nq, samples, seed, beta, s, on,
                                                                  rsq, per, out, status, bd, order);
     else
-      o8_stochastic_kernel<O8_GRAV_GRAD, false><<<g, 128, 0, stream>>>(L, N, queries, cot, nq, samples, seed, beta,
+      o8_stochastic_kernel<O8_GRAV_GRAD, false><<<g, kStochThreads, 0, stream>>>(L, N, queries, cot, nq, samples, seed, beta,
                                                                        s, 0, 0.f, per, out, status, bd, order);
   } else {
     if (softened)
-      o8_stochastic_kernel<O8_SOFT_VJP, true><<<g, 128, 0, stream>>>(L, N, queries, cot, nq, samples, seed, beta, s,
+      o8_stochastic_kernel<O8_SOFT_VJP, true><<<g, kStochThreads, 0, stream>>>(L, N, queries, cot, nq, samples, seed, beta, s,
                                                                      on, rsq, per, out, status, bd, order);
     else
-      o8_stochastic_kernel<O8_GRAV_GRAD_VJP, false><<<g, 128, 0, stream>>>(L, N, queries, cot, nq, samples, seed,
+      o8_stochastic_kernel<O8_GRAV_GRAD_VJP, false><<<g, kStochThreads, 0, stream>>>(L, N, queries, cot, nq, samples, seed,
                                                                            beta, s, 0, 0.f, per, out, status, bd,
                                                                            order);
   }
