@@ -102,9 +102,14 @@ __device__ __forceinline__ int common_levels(uint64_t a, uint64_t b) {
 // ---------------------------------------------------------------------------
 // 1. bounding boxes (per system)
 // ---------------------------------------------------------------------------
-__global__ void bbox_init_kernel(uint32_t* bb, int nseg) {
+// Empty boxes, and [0, n] as the offsets of a single system.
+__global__ void build_init_kernel(uint32_t* bb, int nseg, int64_t* seg_off, int64_t n) {
   int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= nseg) return;
+  if (nseg == 1) {
+    seg_off[0] = 0;
+    seg_off[1] = n;
+  }
   for (int d = 0; d < 3; d++) {
     bb[6 * s + d] = 0xFFFFFFFFu;  // min (ordered)
     bb[6 * s + 3 + d] = 0u;       // max (ordered)
@@ -288,8 +293,13 @@ __device__ __forceinline__ int64_t cell_end(const uint64_t* keys, const uint32_t
 __global__ void emit_nodes_kernel(const uint64_t* __restrict__ keys, const uint32_t* __restrict__ sseg,
                                   const int64_t* __restrict__ sorted_seg_off, int64_t n, const int8_t* __restrict__ dd,
                                   const int8_t* __restrict__ lv, const uint32_t* __restrict__ base,
-                                  NodeRec* __restrict__ nodes, int64_t cap, uint32_t* status) {
+                                  NodeRec* __restrict__ nodes, int64_t cap, uint32_t* __restrict__ meta,
+                                  uint32_t* status) {
   uint32_t total = base[n];
+  if (blockIdx.x == 0 && threadIdx.x == 0) {  // the node count, and whether it exceeds the capacity
+    meta[0] = total <= cap ? total : static_cast<uint32_t>(cap);
+    meta[3] = total > cap ? 1u : 0u;
+  }
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     int d = dd[i];
@@ -567,19 +577,6 @@ __global__ void sseg_kernel(const int64_t* __restrict__ seg_off, int nseg, int64
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x)
     sseg[i] = static_cast<uint32_t>(seg_of(seg_off, nseg, i));
-}
-
-// meta[0] = number of nodes (base[n]); flags an overflow of the capacity.
-__global__ void node_count_kernel(const uint32_t* base, int64_t n, int64_t cap, uint32_t* meta) {
-  uint32_t total = base[n];
-  meta[0] = total <= cap ? total : static_cast<uint32_t>(cap);
-  meta[3] = total > cap ? 1u : 0u;
-}
-
-
-__global__ void single_offsets_kernel(int64_t* seg_off, int64_t n) {
-  seg_off[0] = 0;
-  seg_off[1] = n;
 }
 
 // ---------------------------------------------------------------------------
@@ -1409,8 +1406,10 @@ std::mutex g_reg_mu;
 std::unordered_map<const void*, Header> g_registry;
 
 // Target groups of at most G targets, deepest cells first (group_nodes_kernel).
-cudaError_t cut_groups(cudaStream_t stream, const Layout& L, int64_t n, int nseg, int G, uint32_t* status) {
-  cudaError_t e = cudaMemsetAsync(L.gbins, 0, kGroupBins * sizeof(uint32_t), stream);
+// `zeroed`: gbins is zero already.
+cudaError_t cut_groups(cudaStream_t stream, const Layout& L, int64_t n, int nseg, int G, uint32_t* status,
+                       bool zeroed) {
+  cudaError_t e = zeroed ? cudaSuccess : cudaMemsetAsync(L.gbins, 0, kGroupBins * sizeof(uint32_t), stream);
   if (e != cudaSuccess) return e;
   const unsigned grid = gs(static_cast<int64_t>(L.cap));
   const uint32_t* sseg = nseg > 1 ? L.sseg : nullptr;
@@ -1473,20 +1472,18 @@ int sbh_native_build(cudaStream_t stream, const float* points, const float* mass
   Layout L;
   if (int rc = native_layout(workspace, workspace_bytes, h, L)) return rc;
   uint32_t* status = static_cast<uint32_t*>(workspace);
-  cudaError_t e = cudaMemsetAsync(status, 0, 64, stream);
-  if (e == cudaSuccess) e = cudaMemsetAsync(L.meta, 0, 8 * sizeof(uint32_t), stream);
-  if (e == cudaSuccess) e = cudaMemsetAsync(L.counters, 0, kCounters * sizeof(unsigned long long), stream);
+  // the status word, meta, gbins and counters lead the workspace
+  cudaError_t e = cudaMemsetAsync(
+      status, 0, reinterpret_cast<char*>(L.counters + kCounters) - static_cast<char*>(workspace), stream);
   if (e != cudaSuccess) return fail(SBH_ERR_CUDA, cudaGetErrorString(e));
   // system offsets (device copy, or [0, n] for one system)
   if (num_systems > 1) {
     e = cudaMemcpyAsync(L.seg_off, system_offsets, (num_systems + 1) * sizeof(int64_t), cudaMemcpyDeviceToDevice,
                         stream);
-  } else {
-    single_offsets_kernel<<<1, 1, 0, stream>>>(L.seg_off, n);
   }
   if (e != cudaSuccess) return fail(SBH_ERR_CUDA, cudaGetErrorString(e));
   int nseg = num_systems;
-  bbox_init_kernel<<<(nseg + 255) / 256, 256, 0, stream>>>(L.bb, nseg);
+  build_init_kernel<<<(nseg + 255) / 256, 256, 0, stream>>>(L.bb, nseg, L.seg_off, n);
   if (n > 0) bbox_kernel<<<gs(n), 256, 0, stream>>>(points, n, L.seg_off, nseg, L.bb);
   bbox_finalize_kernel<<<(nseg + 255) / 256, 256, 0, stream>>>(L.bb, nseg, L.seg_off, L.boxes);
   const uint32_t* perm = L.v0;
@@ -1526,8 +1523,8 @@ int sbh_native_build(cudaStream_t stream, const float* points, const float* mass
     slots_kernel<<<gs(n), 256, 0, stream>>>(L.cl, L.dd, n, leaf_size, L.lv, L.base);
     e = exclusive_scan<uint32_t>(stream, ArrayLoad<uint32_t>{L.base}, n, L.base, L.scan_tmp, true);
     if (e != cudaSuccess) return fail(SBH_ERR_CUDA, cudaGetErrorString(e));
-    emit_nodes_kernel<<<gs(n), 256, 0, stream>>>(L.k0, sseg, L.seg_off, n, L.dd, L.lv, L.base, L.nodes, L.cap, status);
-    node_count_kernel<<<1, 1, 0, stream>>>(L.base, n, L.cap, L.meta);
+    emit_nodes_kernel<<<gs(n), 256, 0, stream>>>(L.k0, sseg, L.seg_off, n, L.dd, L.lv, L.base, L.nodes, L.cap, L.meta,
+                                                status);
     gather_particles_kernel<<<gs(n), 256, 0, stream>>>(points, masses, normals, perm, n, L.sp, L.sn);
     e = exclusive_scan<DVec<10>>(stream, MomentLoad{L.sp, sseg, L.boxes}, n, L.P, L.ptmp, true);
     if (e == cudaSuccess && normals)
@@ -1542,7 +1539,7 @@ int sbh_native_build(cudaStream_t stream, const float* points, const float* mass
   // system roots and target groups (meta[1] counts the groups)
   roots_kernel<<<nseg, 32, 0, stream>>>(L.seg_off, nseg, L.base, L.cap, L.roots);
   if (n > 0) {
-    cudaError_t ge = cut_groups(stream, L, n, nseg, kGroup, status);
+    cudaError_t ge = cut_groups(stream, L, n, nseg, kGroup, status, true);
     if (ge != cudaSuccess) return fail(SBH_ERR_CUDA, cudaGetErrorString(ge));
   }
   if (int rc = check_launch("sbh_native_build")) return rc;
@@ -1745,7 +1742,7 @@ int sbh_native_set_group_size(cudaStream_t stream, void* workspace, size_t works
   if (h.n == 0) return SBH_OK;
   // the stats keep describing the last walk: count it on its own groups first
   if (int rc = refresh_counts(stream, workspace, h, L)) return rc;
-  cudaError_t e = cut_groups(stream, L, h.n, h.nseg, group_size, static_cast<uint32_t*>(workspace));
+  cudaError_t e = cut_groups(stream, L, h.n, h.nseg, group_size, static_cast<uint32_t*>(workspace), false);
   if (e != cudaSuccess) return fail(SBH_ERR_CUDA, cudaGetErrorString(e));
   {
     std::lock_guard<std::mutex> lk(g_reg_mu);

@@ -8,6 +8,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 
 namespace sbh {
@@ -168,6 +169,32 @@ __global__ void __launch_bounds__(kScanThreads) scan_tile_apply(Load load, int64
   }
 }
 
+// A few tiles in one block and one launch, the running total carried along.
+constexpr int64_t kScanFewTiles = 8;
+template <typename T, typename Load>
+__global__ void __launch_bounds__(kScanThreads) scan_few_tiles(Load load, int64_t n, T* out, int write_total) {
+  constexpr int kItems = ScanCfg<T>::kItems;
+  T carry = zero_t<T>();
+  for (int64_t tile0 = 0; tile0 < n || tile0 == 0; tile0 += ScanCfg<T>::kTile) {
+    T items[kItems];
+    T acc = zero_t<T>();
+    for (int k = 0; k < kItems; k++) {
+      const int64_t i = tile0 + static_cast<int64_t>(threadIdx.x) * kItems + k;
+      items[k] = i < n ? load(i) : zero_t<T>();
+      acc = acc + items[k];
+    }
+    T tot;
+    T run = carry + block_exclusive(acc, &tot);
+    for (int k = 0; k < kItems; k++) {
+      const int64_t i = tile0 + static_cast<int64_t>(threadIdx.x) * kItems + k;
+      if (i < n) out[i] = run;
+      run = run + items[k];
+    }
+    carry = carry + tot;
+  }
+  if (write_total && threadIdx.x == 0) out[n] = carry;
+}
+
 // Number of tiles (= temporaries of type T) of a scan over n elements of T.
 template <typename T = uint32_t>
 inline int64_t scan_tiles(int64_t n) {
@@ -180,6 +207,10 @@ template <typename T, typename Load>
 cudaError_t exclusive_scan(cudaStream_t s, Load load, int64_t n, T* out, T* tmp,
                            bool write_total) {
   int64_t nt = scan_tiles<T>(n);
+  if (nt <= kScanFewTiles) {
+    scan_few_tiles<T, Load><<<1, kScanThreads, 0, s>>>(load, n, out, write_total ? 1 : 0);
+    return cudaGetLastError();
+  }
   scan_tile_totals<T, Load><<<static_cast<unsigned>(nt), kScanThreads, 0, s>>>(load, n, tmp);
   scan_tile_offsets<T><<<1, kScanThreads, 0, s>>>(tmp, nt);
   scan_tile_apply<T, Load><<<static_cast<unsigned>(nt), kScanThreads, 0, s>>>(
@@ -199,6 +230,20 @@ struct ArrayLoad {
 constexpr int kSortThreads = 256;
 constexpr int kSortRounds = 8;
 constexpr int kSortTile = kSortThreads * kSortRounds;  // 2048 keys per block
+
+// The lanes whose 8-bit digit equals this lane's, among the valid ones: eight
+// ballots. (__match_any_sync runs once per distinct value, some thirty times for
+// random digits: radix_scatter's rounds took about 2 us each with it.)
+__device__ __forceinline__ uint32_t match_digit(uint32_t d, bool valid) {
+  uint32_t peers = __ballot_sync(0xffffffffu, valid);
+#pragma unroll
+  for (int b = 0; b < 8; b++) {
+    const bool one = (d >> b) & 1u;
+    const uint32_t v = __ballot_sync(0xffffffffu, one);
+    peers &= one ? v : ~v;
+  }
+  return peers;
+}
 
 template <typename K>
 __global__ void __launch_bounds__(kSortThreads) radix_count(const K* keys, int64_t n, int shift,
@@ -234,8 +279,8 @@ __global__ void __launch_bounds__(kSortThreads) radix_scatter(const K* keys_in, 
     int64_t i = t0 + r * kSortThreads + threadIdx.x;
     bool valid = i < n;
     K key = valid ? keys_in[i] : K(0);
-    uint32_t d = valid ? (static_cast<uint32_t>(key >> shift) & 255u) : 256u;
-    uint32_t peers = __match_any_sync(0xffffffffu, d);
+    uint32_t d = static_cast<uint32_t>(key >> shift) & 255u;
+    uint32_t peers = match_digit(d, valid);
     uint32_t my = __popc(peers & lanemask_lt);
     if (valid && my == 0) wcnt[warp][d] = __popc(peers);
     __syncthreads();
@@ -261,6 +306,139 @@ __global__ void __launch_bounds__(kSortThreads) radix_scatter(const K* keys_in, 
   }
 }
 
+// Small sorts run in one block: the keys and their input indices stay in
+// registers and shared memory through all the passes, so a sort is one launch
+// where the device-wide passes take five each (10,000 63-bit keys: 40 launches,
+// about 200 us of kernels of 3 to 16 us, bound by launches and by the few blocks'
+// barriers). Each warp holds a contiguous run of the keys, ranks it 32 at a
+// time with ballots against its own digit counters, and one scan over the
+// warps' counters turns ranks into positions; the order of equal digits is kept
+// throughout.
+constexpr int kSmallSortThreads = 1024;
+constexpr int kSmallSortItems = 16;
+constexpr int64_t kSmallSortMax = kSmallSortThreads * kSmallSortItems;  // payloads are 16-bit there
+
+template <typename K>
+struct SmallSortShared {
+  K key[kSmallSortMax];
+  uint16_t val[kSmallSortMax];
+  uint16_t cnt[32][256];
+  uint32_t warp_tot[8];
+};
+
+template <typename K>
+__global__ void __launch_bounds__(kSmallSortThreads, 1)
+    radix_small(K* __restrict__ keys, uint32_t* __restrict__ vals, int n, int bits, int vals_given) {
+  extern __shared__ uint4 small_sort_smem[];
+  SmallSortShared<K>& S = *reinterpret_cast<SmallSortShared<K>*>(small_sort_smem);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int per = (n + 1023) / 1024;  // rounds of 32 keys per warp
+  const int first = warp * 32 * per;
+  const uint32_t lt = (1u << lane) - 1u;
+  K key[kSmallSortItems];
+  uint16_t val[kSmallSortItems];
+#pragma unroll
+  for (int r = 0; r < kSmallSortItems; r++) {
+    const int i = first + 32 * r + lane;
+    key[r] = r < per && i < n ? keys[i] : K(0);
+    val[r] = static_cast<uint16_t>(i);
+  }
+  for (int shift = 0; shift < bits; shift += 8) {
+    for (int d = lane; d < 128; d += 32) reinterpret_cast<uint32_t*>(S.cnt[warp])[d] = 0u;
+    __syncwarp();
+    uint16_t rank[kSmallSortItems];
+#pragma unroll
+    for (int r = 0; r < kSmallSortItems; r++) {
+      if (r < per) {  // uniform
+        const bool in = first + 32 * r + lane < n;
+        const uint32_t d = static_cast<uint32_t>(key[r] >> shift) & 255u;
+        const uint32_t peers = match_digit(d, in);
+        const uint32_t before = in ? S.cnt[warp][d] : 0u;
+        rank[r] = static_cast<uint16_t>(before + __popc(peers & lt));
+        __syncwarp();
+        if (in && (peers & lt) == 0) S.cnt[warp][d] = static_cast<uint16_t>(before + __popc(peers));
+        __syncwarp();
+      }
+    }
+    __syncthreads();
+    // thread d < 256: digit d's count per warp -> first position per warp
+    uint32_t run = 0, inc = 0;
+    if (threadIdx.x < 256) {
+      for (int w = 0; w < 32; w++) run += S.cnt[w][threadIdx.x];
+      inc = run;
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += v;
+      }
+      if (lane == 31) S.warp_tot[warp] = inc;
+    }
+    __syncthreads();
+    if (threadIdx.x < 256) {
+      uint32_t at = inc - run;
+      for (int w = 0; w < warp; w++) at += S.warp_tot[w];
+      for (int w = 0; w < 32; w++) {
+        const uint32_t c = S.cnt[w][threadIdx.x];
+        S.cnt[w][threadIdx.x] = static_cast<uint16_t>(at);
+        at += c;
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kSmallSortItems; r++) {
+      if (r < per && first + 32 * r + lane < n) {
+        const uint32_t d = static_cast<uint32_t>(key[r] >> shift) & 255u;
+        const int p = S.cnt[warp][d] + rank[r];
+        S.key[p] = key[r];
+        S.val[p] = val[r];
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kSmallSortItems; r++) {
+      const int i = first + 32 * r + lane;
+      if (r < per && i < n) {
+        key[r] = S.key[i];
+        val[r] = S.val[i];
+      }
+    }
+    __syncthreads();
+  }
+  uint32_t out[kSmallSortItems];
+#pragma unroll
+  for (int r = 0; r < kSmallSortItems; r++) {
+    const int i = first + 32 * r + lane;
+    if (r < per && i < n) out[r] = vals_given ? vals[val[r]] : val[r];
+  }
+  __syncthreads();  // the given payloads are read before any is overwritten
+#pragma unroll
+  for (int r = 0; r < kSmallSortItems; r++) {
+    const int i = first + 32 * r + lane;
+    if (r < per && i < n) {
+      keys[i] = key[r];
+      vals[i] = out[r];
+    }
+  }
+}
+
+template <typename K>
+cudaError_t radix_sort_small(cudaStream_t s, K* keys, uint32_t* vals, int64_t n, int bits, bool vals_given) {
+  static std::atomic<uint64_t> ready[2];  // devices whose copy of the kernel may take this much shared memory
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const uint64_t bit = 1ull << (dev & 63);
+  std::atomic<uint64_t>& r = ready[(dev >> 6) & 1];
+  if (!(r.load() & bit)) {
+    e = cudaFuncSetAttribute(radix_small<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             static_cast<int>(sizeof(SmallSortShared<K>)));
+    if (e != cudaSuccess) return e;
+    r.fetch_or(bit);
+  }
+  radix_small<K><<<1, kSmallSortThreads, sizeof(SmallSortShared<K>), s>>>(keys, vals, static_cast<int>(n), bits,
+                                                                         vals_given ? 1 : 0);
+  return cudaGetLastError();
+}
+
 inline int64_t radix_blocks(int64_t n) { return n <= 0 ? 1 : (n + kSortTile - 1) / kSortTile; }
 
 // Workspace elements (u32) for radix_sort's histogram + scan temporaries.
@@ -280,6 +458,10 @@ cudaError_t radix_sort(cudaStream_t s, K* k0, uint32_t* v0, K* k1, uint32_t* v1,
   if (n <= 0) {
     *which = 0;
     return cudaSuccess;
+  }
+  if (n <= kSmallSortMax && bits > 0) {
+    *which = 0;
+    return radix_sort_small<K>(s, k0, v0, n, bits, vals_given);
   }
   for (int shift = 0; shift < bits; shift += 8) {
     K* kin = cur == 0 ? k0 : k1;
