@@ -27,6 +27,22 @@ __device__ __forceinline__ float vrsqrt(float a) {
 }
 __device__ __forceinline__ float2 vrsqrt(float2 a) { return make_float2(vrsqrt(a.x), vrsqrt(a.y)); }
 
+// 1 / a and 2^a by the special-function unit (a few ulps; normal arguments).
+__device__ __forceinline__ float vrcp(float a) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+  return r;
+}
+__device__ __forceinline__ float2 vrcp(float2 a) { return make_float2(vrcp(a.x), vrcp(a.y)); }
+__device__ __forceinline__ float vexp2(float a) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+  return r;
+}
+__device__ __forceinline__ float2 vexp2(float2 a) { return make_float2(vexp2(a.x), vexp2(a.y)); }
+__device__ __forceinline__ float vneg(float a) { return -a; }
+__device__ __forceinline__ float2 vneg(float2 a) { return make_float2(-a.x, -a.y); }
+
 template <typename V>
 __device__ __forceinline__ V vsplat(float s);
 template <>
