@@ -765,47 +765,6 @@ __device__ __forceinline__ void lq_node_adjoint(const float* x, const float* S, 
   }
 }
 
-constexpr int kTile = 32;  // node records staged at once (the stochastic kernels)
-
-// Bulk copies (the TMA unit's non-tensor cp.async.bulk, no multicast) into
-// shared memory, completed on an mbarrier. The waits are bounded: a copy
-// that never completes makes the wait return false, and the caller flags
-// the workspace's status word and stops instead of spinning.
-__device__ __forceinline__ unsigned smem_addr(const void* p) {
-  return static_cast<unsigned>(__cvta_generic_to_shared(p));
-}
-
-__device__ __forceinline__ void mbar_init(uint64_t* bar) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_addr(bar)) : "memory");
-  asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-}
-
-// Issued by one lane: orders the warp's earlier reads of the destination
-// (generic proxy) before the copy's writes (async proxy), arms the barrier
-// for `bytes` and starts the copy. dst, src and bytes are multiples of 16.
-__device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, unsigned bytes, uint64_t* bar) {
-  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_addr(bar)), "r"(bytes)
-               : "memory");
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
-                   smem_addr(dst)),
-               "l"(src), "r"(bytes), "r"(smem_addr(bar))
-               : "memory");
-}
-
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t phase) {
-  for (int i = 0; i < (1 << 22); i++) {
-    uint32_t done;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(done)
-        : "r"(smem_addr(bar)), "r"(phase)
-        : "memory");
-    if (done) return true;
-  }
-  return false;
-}
-
 // Group centre and squared half diagonal, IEEE operations in the oracle's
 // order (group_centre in oracle/sbh_oracle.c), so both take the same
 // linearization decisions.
@@ -864,6 +823,13 @@ struct WalkQueues {
   uint32_t group;
 };
 
+// Per work item a tag that it hands down the tree (the stochastic estimator's
+// coefficients).
+template <int W>
+struct WalkTags {
+  uint16_t stack[WalkQueues<W>::kStack], quad[64 * W], leaf[64 * W];
+};
+
 // One warp's share: the staged sources of its batch, their indices, its sums
 // of the linearized quadrupoles (a_q (3), J (6) per lane) and, for the
 // adjoint, the group's cotangent sums (W (3), V (6)) and the reduction buffer.
@@ -879,6 +845,7 @@ struct WarpShared<true> {
   float4 stage[96];
   float4 red[8 * kRedStride];
   int idx[32];
+  float coef[32];  // scaled batches: the sources' coefficients
   float acc[9][32];
   float wv[12];
 };
@@ -902,6 +869,74 @@ __device__ __forceinline__ uint32_t coop_next_group(const WalkTargets& G, WalkQu
 struct Frontier {
   int top, nfar, nquad, nleaf;
 };
+
+// Appends what the lanes found to the lists and the stack (m entries were
+// taken off it), in warp order, and moves the frontier's state on.
+template <int W, bool QUAD, bool TAG>
+__device__ __forceinline__ void frontier_put(WalkQueues<W>& q, Frontier& f, int m, int k, bool far, bool lin, bool quad,
+                                             bool leaf, const int2& range, const int4& c0, const int4& c1,
+                                             uint16_t tag, uint16_t quad_tag, WalkTags<W>* tags, int warp, int lane) {
+  const int nc = (c0.x >= 0) + (c0.y >= 0) + (c0.z >= 0) + (c0.w >= 0) + (c1.x >= 0) + (c1.y >= 0) + (c1.z >= 0) +
+                 (c1.w >= 0);
+  const uint32_t lt = (1u << lane) - 1u;
+  const uint32_t bf = __ballot_sync(0xffffffffu, far), bl = __ballot_sync(0xffffffffu, leaf);
+  const uint32_t bq = QUAD ? __ballot_sync(0xffffffffu, quad) : 0u;
+  int inc = nc;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += v;
+  }
+  const int total = __shfl_sync(0xffffffffu, inc, 31);
+  int4 at = make_int4(f.nfar, f.nquad, f.nleaf, f.top - m);  // the warp's first positions
+  int4 sum = make_int4(__popc(bf), __popc(bq), __popc(bl), total);
+  if (lane == 0) q.cnt[warp] = sum;
+  __syncthreads();  // also: every warp has read its stack entries
+  sum = make_int4(0, 0, 0, 0);
+  for (int w = 0; w < W; w++) {
+    const int4 c = q.cnt[w];
+    if (w < warp) {
+      at.x += c.x;
+      at.y += c.y;
+      at.z += c.z;
+      at.w += c.w;
+    }
+    sum.x += c.x;
+    sum.y += c.y;
+    sum.z += c.z;
+    sum.w += c.w;
+  }
+  if (far) q.far[at.x + __popc(bf & lt)] = lin ? (k | INT_MIN) : k;
+  if (QUAD && quad) {
+    const int i = at.y + __popc(bq & lt);
+    q.quad[i] = k;
+    if (TAG) tags->quad[i] = quad_tag;
+  }
+  if (leaf) {
+    const int i = at.z + __popc(bl & lt);
+    q.leaf[i] = range;
+    if (TAG) tags->leaf[i] = tag;
+  }
+  if (nc > 0) {
+    const int i = at.w + inc - nc;
+    int* s = q.stack + i;
+    s[0] = c0.x;
+    if (c0.y >= 0) s[1] = c0.y;
+    if (c0.z >= 0) s[2] = c0.z;
+    if (c0.w >= 0) s[3] = c0.w;
+    if (c1.x >= 0) s[4] = c1.x;
+    if (c1.y >= 0) s[5] = c1.y;
+    if (c1.z >= 0) s[6] = c1.z;
+    if (c1.w >= 0) s[7] = c1.w;
+    if (TAG)
+      for (int c = 0; c < nc; c++) tags->stack[i + c] = tag;
+  }
+  f.top += sum.w - m;
+  f.nfar += sum.x;
+  f.nquad += sum.y;
+  f.nleaf += sum.z;
+  __syncthreads();
+}
 
 enum { kActDone = 0, kActStep = 1, kActFar = 2, kActQuad = 3, kActLeaf = 4 };
 
@@ -956,13 +991,15 @@ __device__ __forceinline__ LeafShare leaf_share(const int2* leaf, int cnt, int l
   return s;
 }
 
-// The particle at the run's position b + lane, or -1 past its end. Leaves
-// hold at least one particle, so their first positions are distinct.
-__device__ __forceinline__ int leaf_particle(const LeafShare& s, int b, int lane) {
+// The particle at the run's position b + lane, or -1 past its end; *of: the lane
+// that holds its leaf. Leaves hold at least one particle, so their first
+// positions are distinct.
+__device__ __forceinline__ int leaf_particle(const LeafShare& s, int b, int lane, int* of = nullptr) {
   const int before = __popc(__ballot_sync(0xffffffffu, s.valid && s.excl < b));
   const bool here = s.valid && s.excl >= b && s.excl < b + 32;
   const uint32_t heads = __reduce_or_sync(0xffffffffu, here ? 1u << (s.excl - b) : 0u);
   const int l = before + __popc(heads & (0xffffffffu >> (31 - lane))) - 1;
+  if (of) *of = l & 31;
   const int start = __shfl_sync(0xffffffffu, s.start, l & 31), excl = __shfl_sync(0xffffffffu, s.excl, l & 31);
   return b + lane < s.total ? start + b + lane - excl : -1;
 }
@@ -1463,7 +1500,7 @@ int sbh_native_build(cudaStream_t stream, const float* points, const float* mass
   if (leaf_size < 1 || leaf_size > 32) return invalid("leaf_size must be in [1, 32]");
   if (n > 0 && (!points || !masses)) return invalid("points and masses must be non-null");
   if (!workspace) return fail(SBH_ERR_WORKSPACE, "workspace is null");
-  // the node records are read with 16-byte vector loads and bulk copies
+  // the node records are read with 16-byte vector loads
   if (reinterpret_cast<uintptr_t>(workspace) % 16 != 0) return invalid("workspace must be 16-byte aligned");
   size_t need = sbh_native_workspace_bytes(n, num_systems, leaf_size, normals != nullptr, with_adjoint);
   if (workspace_bytes < need)
@@ -1647,6 +1684,19 @@ cudaError_t launch_coop(cudaStream_t stream, uint32_t* counter, int64_t max_grou
   constexpr size_t kSmem = sizeof(CoopShared<W, ADJ>);
   const unsigned blocks = walk_blocks(kernel, max_groups, 1, 32 * W, kSmem);
   kernel<<<blocks, 32 * W, kSmem, stream>>>(args...);
+  return cudaGetLastError();
+}
+
+template <bool ADJ>
+cudaError_t launch_stochastic(cudaStream_t stream, const Layout& L, const Header& h, float beta_c, float beta_f,
+                              float eps2, int samples, uint64_t seed, const float* cot, float* out) {
+  cudaError_t e = cudaMemsetAsync(L.work, 0, sizeof(uint32_t), stream);
+  if (e != cudaSuccess) return e;
+  constexpr size_t kSmem = sizeof(StochShared<ADJ>);
+  const unsigned blocks = walk_blocks(stoch_kernel<ADJ>, h.n + h.nseg, 1, 32 * kStochWarps, kSmem);
+  stoch_kernel<ADJ><<<blocks, 32 * kStochWarps, kSmem, stream>>>(tree_view(L), self_targets(L, h), beta_c, beta_f, eps2,
+                                                                 samples, seed, cot, out, L.gq, L.node_adj,
+                                                                 L.part_adj);
   return cudaGetLastError();
 }
 
@@ -1875,11 +1925,9 @@ int sbh_native_stochastic_force(cudaStream_t stream, const sbh_native_params* pa
   if (!force_out) return invalid("force_out must be non-null");
   if (partial_range(h)) return invalid("the stochastic estimator needs the full target range");
   const WalkParams wp = walk_params(params);
-  uint32_t* status = static_cast<uint32_t*>(workspace);  // SBH_DEV_ITER_LIMIT if a tile copy never completes
-  cudaError_t e = cudaMemsetAsync(status, 0, sizeof(uint32_t), stream);
+  cudaError_t e = cudaMemsetAsync(workspace, 0, sizeof(uint32_t), stream);  // the status word
   if (e == cudaSuccess)
-    e = launch_walk(stream, L.work, h.n + h.nseg, stoch_group_kernel, tree_view(L), self_targets(L, h), beta_coarse,
-                    params->beta, wp.eps2, samples, seed, force_out, status);
+    e = launch_stochastic<false>(stream, L, h, beta_coarse, params->beta, wp.eps2, samples, seed, nullptr, force_out);
   if (e != cudaSuccess) return fail(SBH_ERR_CUDA, cudaGetErrorString(e));
   remember_walk(workspace, 0, nullptr);
   return check_launch("sbh_native_stochastic_force");
@@ -1913,12 +1961,9 @@ int sbh_native_stochastic_force_vjp(cudaStream_t stream, const sbh_native_params
   if (e != cudaSuccess) return fail(SBH_ERR_CUDA, cudaGetErrorString(e));
   zero_node_adj_kernel<<<gs(L.cap * kNodeAdj), 256, 0, stream>>>(L.node_adj, L.meta);
   const WalkParams wp = walk_params(params);
-  uint32_t* status = static_cast<uint32_t*>(workspace);
-  if (!force_out) e = cudaMemsetAsync(status, 0, sizeof(uint32_t), stream);  // else the forward cleared it
+  if (!force_out) e = cudaMemsetAsync(workspace, 0, sizeof(uint32_t), stream);  // else the forward cleared it
   if (e == cudaSuccess)
-    e = launch_walk(stream, L.work, h.n + h.nseg, stoch_adjoint_kernel, tree_view(L), self_targets(L, h),
-                    beta_coarse, params->beta, wp.eps2, samples, seed, cotangent, L.gq, L.node_adj, L.part_adj,
-                    status);
+    e = launch_stochastic<true>(stream, L, h, beta_coarse, params->beta, wp.eps2, samples, seed, cotangent, nullptr);
   if (e != cudaSuccess) return fail(SBH_ERR_CUDA, cudaGetErrorString(e));
   remember_walk(workspace, 0, nullptr);
   return sbh_native_adjoint_finalize(stream, grad_points, grad_masses, workspace, workspace_bytes);
