@@ -1622,7 +1622,8 @@ static void o8_launch_warp_kind(int warps, cudaStream_t stream, const Leaf3* L, 
 // Eight warps share 32 queries while the query sets alone give the SMs fewer
 // than 16 warps each (75,776 queries) and the sums are taken in units; else each
 // warp has its own queries and the caller's `threads` gives the warps per block
-// (at most 8: the result does not depend on it). Softened force / VJP of the
+// (at most 4, so that a block's slowest warp holds up few others: 10^5 queries 7.7
+// / 8.5 ms against 8.2 / 9.5 with 8; the result does not depend on it). Softened force / VJP of the
 // particles themselves, ms on a B200, shared against own: 5,000 particles 0.55 /
 // 0.56 and 2.5 / 2.6 (3.1 / 3.1 before the next node's prefetch), 20,000 1.6 / 1.6
 // and 4.2 / 4.3, 60,000 in a uniform cube 5.6 / 5.8 and 6.7 / 6.9, in a Plummer
@@ -1634,7 +1635,7 @@ static void o8_launch_warp_sets(int threads, int64_t nq, uint32_t leaves, cudaSt
   if (o8_shared_sets(nq, leaves)) {
     o8_launch_warp_kind<KERNEL, STACK, 8>(8, stream, args...);
   } else {
-    const int warps = threads >= 64 ? (threads < 256 ? threads / 32 : 8) : 1;
+    const int warps = threads >= 64 ? (threads < 128 ? threads / 32 : 4) : 1;
     o8_launch_warp_kind<KERNEL, STACK, 1>(warps, stream, args...);
   }
 }
