@@ -260,49 +260,59 @@ __global__ void __launch_bounds__(kSortThreads) radix_count(const K* keys, int64
   hist[static_cast<int64_t>(threadIdx.x) * nblocks + blockIdx.x] = h[threadIdx.x];
 }
 
+// Each warp ranks its contiguous run of 256 keys, 32 at a time, against its own
+// digit counters without waiting for the others; one scan over the warps'
+// counters then places them. (Ranking 256 keys per round across the block took
+// five barriers a round, about 40 per tile.)
 template <typename K>
 __global__ void __launch_bounds__(kSortThreads) radix_scatter(const K* keys_in, const uint32_t* vals_in,
                                                               K* keys_out, uint32_t* vals_out,
                                                               int64_t n, int shift,
                                                               const uint32_t* hist_off,
                                                               int64_t nblocks) {
-  __shared__ uint32_t goff[256];
-  __shared__ uint32_t wcnt[kSortThreads / 32][256];
-  __shared__ uint32_t rtot[256];
-  int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  goff[threadIdx.x] = hist_off[static_cast<int64_t>(threadIdx.x) * nblocks + blockIdx.x];
-  for (int w = 0; w < kSortThreads / 32; w++) wcnt[w][threadIdx.x] = 0;
-  __syncthreads();
-  int64_t t0 = static_cast<int64_t>(blockIdx.x) * kSortTile;
-  uint32_t lanemask_lt = (1u << lane) - 1u;
+  constexpr int kWarps = kSortThreads / 32;
+  __shared__ uint32_t cnt[kWarps][256];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t goff = hist_off[static_cast<int64_t>(threadIdx.x) * nblocks + blockIdx.x];
+  for (int d = lane; d < 256; d += 32) cnt[warp][d] = 0;
+  __syncwarp();
+  const int64_t first = static_cast<int64_t>(blockIdx.x) * kSortTile + warp * (32 * kSortRounds) + lane;
+  const uint32_t lt = (1u << lane) - 1u;
+  K key[kSortRounds];
+  uint32_t val[kSortRounds], rank[kSortRounds];
+#pragma unroll
   for (int r = 0; r < kSortRounds; r++) {
-    int64_t i = t0 + r * kSortThreads + threadIdx.x;
-    bool valid = i < n;
-    K key = valid ? keys_in[i] : K(0);
-    uint32_t d = static_cast<uint32_t>(key >> shift) & 255u;
-    uint32_t peers = match_digit(d, valid);
-    uint32_t my = __popc(peers & lanemask_lt);
-    if (valid && my == 0) wcnt[warp][d] = __popc(peers);
-    __syncthreads();
-    {
-      uint32_t s = 0;
-      for (int w = 0; w < kSortThreads / 32; w++) {
-        uint32_t c = wcnt[w][threadIdx.x];
-        wcnt[w][threadIdx.x] = s;
-        s += c;
-      }
-      rtot[threadIdx.x] = s;
+    const int64_t i = first + 32 * r;
+    key[r] = i < n ? keys_in[i] : K(0);
+    val[r] = i < n ? (vals_in ? vals_in[i] : static_cast<uint32_t>(i)) : 0u;
+  }
+#pragma unroll
+  for (int r = 0; r < kSortRounds; r++) {
+    const bool valid = first + 32 * r < n;
+    const uint32_t d = static_cast<uint32_t>(key[r] >> shift) & 255u;
+    const uint32_t peers = match_digit(d, valid);
+    const uint32_t before = cnt[warp][d];
+    rank[r] = before + __popc(peers & lt);
+    __syncwarp();
+    if (valid && (peers & lt) == 0) cnt[warp][d] = before + __popc(peers);
+    __syncwarp();
+  }
+  __syncthreads();
+  uint32_t at = goff;  // thread d: digit d's first position per warp
+#pragma unroll
+  for (int w = 0; w < kWarps; w++) {
+    const uint32_t c = cnt[w][threadIdx.x];
+    cnt[w][threadIdx.x] = at;
+    at += c;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < kSortRounds; r++) {
+    if (first + 32 * r < n) {
+      const uint32_t dst = cnt[warp][static_cast<uint32_t>(key[r] >> shift) & 255u] + rank[r];
+      keys_out[dst] = key[r];
+      vals_out[dst] = val[r];
     }
-    __syncthreads();
-    if (valid) {
-      uint32_t dst = goff[d] + wcnt[warp][d] + my;
-      keys_out[dst] = key;
-      vals_out[dst] = vals_in ? vals_in[i] : static_cast<uint32_t>(i);
-    }
-    __syncthreads();
-    goff[threadIdx.x] += rtot[threadIdx.x];
-    for (int w = 0; w < kSortThreads / 32; w++) wcnt[w][threadIdx.x] = 0;
-    __syncthreads();
   }
 }
 
@@ -316,6 +326,7 @@ __global__ void __launch_bounds__(kSortThreads) radix_scatter(const K* keys_in, 
 // throughout.
 constexpr int kSmallSortThreads = 1024;
 constexpr int kSmallSortItems = 16;
+constexpr int kSmallSortRun = 8;
 constexpr int64_t kSmallSortMax = kSmallSortThreads * kSmallSortItems;  // payloads are 16-bit there
 
 template <typename K>
@@ -336,60 +347,100 @@ __global__ void __launch_bounds__(kSmallSortThreads, 1)
   const int first = warp * 32 * per;
   const uint32_t lt = (1u << lane) - 1u;
   K key[kSmallSortItems];
-  uint16_t val[kSmallSortItems];
-#pragma unroll
-  for (int r = 0; r < kSmallSortItems; r++) {
-    const int i = first + 32 * r + lane;
-    key[r] = r < per && i < n ? keys[i] : K(0);
-    val[r] = static_cast<uint16_t>(i);
-  }
-  for (int shift = 0; shift < bits; shift += 8) {
-    for (int d = lane; d < 128; d += 32) reinterpret_cast<uint32_t*>(S.cnt[warp])[d] = 0u;
-    __syncwarp();
-    uint16_t rank[kSmallSortItems];
+  uint32_t val[kSmallSortItems];  // input index, and above it the rank within the pass
+  // Keys of more than 32 bits are first sorted by their top 32 alone, half the
+  // passes. Few keys of so small a set agree in those, and their runs are then
+  // ordered in place; a run of more than kSmallSortRun keys (coincident points)
+  // sends the sort back to all bits.
+  for (int low = sizeof(K) > 4 && bits > 32 ? bits - 32 : 0;; low = 0) {
 #pragma unroll
     for (int r = 0; r < kSmallSortItems; r++) {
-      if (r < per) {  // uniform
-        const bool in = first + 32 * r + lane < n;
-        const uint32_t d = static_cast<uint32_t>(key[r] >> shift) & 255u;
-        const uint32_t peers = match_digit(d, in);
-        const uint32_t before = in ? S.cnt[warp][d] : 0u;
-        rank[r] = static_cast<uint16_t>(before + __popc(peers & lt));
-        __syncwarp();
-        if (in && (peers & lt) == 0) S.cnt[warp][d] = static_cast<uint16_t>(before + __popc(peers));
-        __syncwarp();
-      }
+      const int i = first + 32 * r + lane;
+      key[r] = r < per && i < n ? keys[i] : K(0);
+      val[r] = static_cast<uint32_t>(i) & 0xFFFFu;
     }
-    __syncthreads();
-    // thread d < 256: digit d's count per warp -> first position per warp
-    uint32_t run = 0, inc = 0;
-    if (threadIdx.x < 256) {
-      for (int w = 0; w < 32; w++) run += S.cnt[w][threadIdx.x];
-      inc = run;
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t v = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += v;
-      }
-      if (lane == 31) S.warp_tot[warp] = inc;
-    }
-    __syncthreads();
-    if (threadIdx.x < 256) {
-      uint32_t at = inc - run;
-      for (int w = 0; w < warp; w++) at += S.warp_tot[w];
-      for (int w = 0; w < 32; w++) {
-        const uint32_t c = S.cnt[w][threadIdx.x];
-        S.cnt[w][threadIdx.x] = static_cast<uint16_t>(at);
-        at += c;
-      }
-    }
-    __syncthreads();
+    for (int shift = low; shift < bits; shift += 8) {
+      for (int d = lane; d < 128; d += 32) reinterpret_cast<uint32_t*>(S.cnt[warp])[d] = 0u;
+      __syncwarp();
 #pragma unroll
-    for (int r = 0; r < kSmallSortItems; r++) {
-      if (r < per && first + 32 * r + lane < n) {
-        const uint32_t d = static_cast<uint32_t>(key[r] >> shift) & 255u;
-        const int p = S.cnt[warp][d] + rank[r];
-        S.key[p] = key[r];
-        S.val[p] = val[r];
+      for (int r = 0; r < kSmallSortItems; r++) {
+        if (r < per) {  // uniform
+          const bool in = first + 32 * r + lane < n;
+          const uint32_t d = static_cast<uint32_t>(key[r] >> shift) & 255u;
+          const uint32_t peers = match_digit(d, in);
+          const uint32_t before = in ? S.cnt[warp][d] : 0u;
+          val[r] |= (before + __popc(peers & lt)) << 16;
+          __syncwarp();
+          if (in && (peers & lt) == 0) S.cnt[warp][d] = static_cast<uint16_t>(before + __popc(peers));
+          __syncwarp();
+        }
+      }
+      __syncthreads();
+      // thread d < 256: digit d's count per warp -> first position per warp
+      uint32_t run = 0, inc = 0;
+      if (threadIdx.x < 256) {
+        for (int w = 0; w < 32; w++) run += S.cnt[w][threadIdx.x];
+        inc = run;
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint32_t v = __shfl_up_sync(0xffffffffu, inc, o);
+          if (lane >= o) inc += v;
+        }
+        if (lane == 31) S.warp_tot[warp] = inc;
+      }
+      __syncthreads();
+      if (threadIdx.x < 256) {
+        uint32_t at = inc - run;
+        for (int w = 0; w < warp; w++) at += S.warp_tot[w];
+        for (int w = 0; w < 32; w++) {
+          const uint32_t c = S.cnt[w][threadIdx.x];
+          S.cnt[w][threadIdx.x] = static_cast<uint16_t>(at);
+          at += c;
+        }
+      }
+      __syncthreads();
+#pragma unroll
+      for (int r = 0; r < kSmallSortItems; r++) {
+        if (r < per && first + 32 * r + lane < n) {
+          const uint32_t d = static_cast<uint32_t>(key[r] >> shift) & 255u;
+          const int p = static_cast<int>(S.cnt[warp][d] + (val[r] >> 16));
+          S.key[p] = key[r];
+          S.val[p] = static_cast<uint16_t>(val[r]);
+        }
+      }
+      __syncthreads();
+#pragma unroll
+      for (int r = 0; r < kSmallSortItems; r++) {
+        const int i = first + 32 * r + lane;
+        if (r < per && i < n) {
+          key[r] = S.key[i];
+          val[r] = S.val[i];
+        }
+      }
+      __syncthreads();
+    }
+    if (low == 0) break;
+    bool again = false;
+    for (int i = static_cast<int>(threadIdx.x); i < n; i += kSmallSortThreads) {
+      const K top = S.key[i] >> low;
+      if (i > 0 && S.key[i - 1] >> low == top) continue;  // not the head of a run
+      int end = i + 1;
+      while (end < n && end - i <= kSmallSortRun && S.key[end] >> low == top) end++;
+      if (end - i > kSmallSortRun) again = true;
+    }
+    if (__syncthreads_or(again)) continue;
+    for (int i = static_cast<int>(threadIdx.x); i < n; i += kSmallSortThreads) {
+      const K top = S.key[i] >> low;
+      if ((i > 0 && S.key[i - 1] >> low == top) || i + 1 >= n || S.key[i + 1] >> low != top) continue;
+      for (int e = i + 1; e < n && S.key[e] >> low == top; e++) {  // stable insertion
+        const K k = S.key[e];
+        const uint16_t v = S.val[e];
+        int at = e;
+        for (; at > i && S.key[at - 1] > k; at--) {
+          S.key[at] = S.key[at - 1];
+          S.val[at] = S.val[at - 1];
+        }
+        S.key[at] = k;
+        S.val[at] = v;
       }
     }
     __syncthreads();
@@ -401,13 +452,13 @@ __global__ void __launch_bounds__(kSmallSortThreads, 1)
         val[r] = S.val[i];
       }
     }
-    __syncthreads();
+    break;
   }
   uint32_t out[kSmallSortItems];
 #pragma unroll
   for (int r = 0; r < kSmallSortItems; r++) {
     const int i = first + 32 * r + lane;
-    if (r < per && i < n) out[r] = vals_given ? vals[val[r]] : val[r];
+    if (r < per && i < n) out[r] = vals_given ? vals[val[r] & 0xFFFFu] : val[r] & 0xFFFFu;
   }
   __syncthreads();  // the given payloads are read before any is overwritten
 #pragma unroll

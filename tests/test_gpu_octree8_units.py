@@ -62,3 +62,18 @@ def test_sorts_around_the_single_block_limit(cuda, n):
     arr = O.NativeTree(p, m, leaf_size=16).arrays()
     np.testing.assert_array_equal(keys, arr["keys"])
     np.testing.assert_array_equal(perm.astype(np.int64), arr["perm"])
+
+
+@pytest.mark.parametrize("copies", [2, 8, 9, 40])
+def test_small_sorts_with_keys_that_agree_in_their_top_bits(cuda, copies):
+    """Clusters far below the resolution of a key's top 32 bits (about 2^-11 of
+    the box per axis): runs up to the limit of the in-place pass and past it."""
+    rng = np.random.default_rng(copies)
+    centres = rng.random((3000 // copies, 3))
+    p = (np.repeat(centres, copies, axis=0) + rng.uniform(-2e-6, 2e-6, (3000 // copies * copies, 3)))
+    p = p.astype(np.float32)[rng.permutation(3000 // copies * copies)]
+    m = np.full(len(p), 1.0 / len(p), np.float32)
+    keys, perm, _ = B.NativeTree().build(p, m, leaf_size=8).export()
+    arr = O.NativeTree(p, m, leaf_size=8).arrays()
+    np.testing.assert_array_equal(keys, arr["keys"])
+    np.testing.assert_array_equal(perm.astype(np.int64), arr["perm"])
