@@ -272,6 +272,9 @@ __global__ void __launch_bounds__(kSortThreads) radix_scatter(const K* keys_in, 
                                                               int64_t nblocks) {
   constexpr int kWarps = kSortThreads / 32;
   __shared__ uint32_t cnt[kWarps][256];
+  __shared__ uint32_t to[256];  // digit's first position in the output, less its first in the tile
+  __shared__ K skey[kSortTile];
+  __shared__ uint32_t sval[kSortTile];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t goff = hist_off[static_cast<int64_t>(threadIdx.x) * nblocks + blockIdx.x];
   for (int d = lane; d < 256; d += 32) cnt[warp][d] = 0;
@@ -298,7 +301,11 @@ __global__ void __launch_bounds__(kSortThreads) radix_scatter(const K* keys_in, 
     __syncwarp();
   }
   __syncthreads();
-  uint32_t at = goff;  // thread d: digit d's first position per warp
+  uint32_t sum = 0;
+#pragma unroll
+  for (int w = 0; w < kWarps; w++) sum += cnt[w][threadIdx.x];
+  uint32_t at = block_exclusive(sum, static_cast<uint32_t*>(nullptr));  // thread d: digit d's place in the tile
+  to[threadIdx.x] = goff - at;
 #pragma unroll
   for (int w = 0; w < kWarps; w++) {
     const uint32_t c = cnt[w][threadIdx.x];
@@ -309,9 +316,23 @@ __global__ void __launch_bounds__(kSortThreads) radix_scatter(const K* keys_in, 
 #pragma unroll
   for (int r = 0; r < kSortRounds; r++) {
     if (first + 32 * r < n) {
-      const uint32_t dst = cnt[warp][static_cast<uint32_t>(key[r] >> shift) & 255u] + rank[r];
-      keys_out[dst] = key[r];
-      vals_out[dst] = val[r];
+      const uint32_t p = cnt[warp][static_cast<uint32_t>(key[r] >> shift) & 255u] + rank[r];
+      skey[p] = key[r];
+      sval[p] = val[r];
+    }
+  }
+  __syncthreads();
+  // neighbours in the tile's order mostly go to neighbouring places
+  const int64_t left = n - static_cast<int64_t>(blockIdx.x) * kSortTile;
+  const int m = left < kSortTile ? static_cast<int>(left) : kSortTile;
+#pragma unroll
+  for (int r = 0; r < kSortRounds; r++) {
+    const int i = r * kSortThreads + static_cast<int>(threadIdx.x);
+    if (i < m) {
+      const K k = skey[i];
+      const uint32_t dst = to[static_cast<uint32_t>(k >> shift) & 255u] + static_cast<uint32_t>(i);
+      keys_out[dst] = k;
+      vals_out[dst] = sval[i];
     }
   }
 }
