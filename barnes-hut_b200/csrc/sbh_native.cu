@@ -1072,11 +1072,12 @@ __device__ __forceinline__ void lq_eval(const NodeRec* nd, const float4& A, cons
 // serve at more warps per SM. A tree walks with the kernels of its current group
 // size (sbh_native_set_group_size). Measured on a B200, 2^20 particles: force at
 // 4 blocks per SM 9.6 ms, at 5 (96 registers, spilling) 10.1; adjoint at 4 blocks
-// 23.7 ms, at 3 24.6.
+// 23.7 ms, at 3 24.6. Groups of 64 (uniform cube): force at 7 blocks 5.8 ms, at 5
+// 5.9; force + adjoint at 5 blocks 13.5 ms, at 6 14.1, at 7 (spilling) 14.4.
 namespace tpl2 {
 constexpr int kTPL = 2;
 constexpr int kForceWalkMinBlocks = 7;
-constexpr int kAdjointWalkMinBlocks = 7;
+constexpr int kAdjointWalkMinBlocks = 5;
 #include "sbh_native_walks.inc"
 }  // namespace tpl2
 
