@@ -183,36 +183,6 @@ __device__ __forceinline__ float soft_coeff(float r2, float mass, const Soft& s)
   return -mass * att * inv_r3;
 }
 
-// Query-side VJP of the softened force: acc += -m (lin g - rad r).
-__device__ __forceinline__ void soft_vjp_accum(float rx, float ry, float rz, float mass,
-                                               float gx, float gy, float gz, const Soft& s,
-                                               float& ax, float& ay, float& az) {
-  float r2 = rx * rx + ry * ry + rz * rz;
-  float inv_r = rsqrtf(r2 + s.eps * s.eps + 1e-12f);
-  float inv_r3 = inv_r * inv_r * inv_r;
-  float inv_r5 = inv_r3 * inv_r * inv_r;
-  float att = 1.0f;
-  float cc = 0.0f;
-  // below kAttUnityU (r^2 under unity_r2): att = 1, and cc = ir3 r e / (2 sqrt(pi) cutoff^3) is
-  // below 1e-4 (r^2 + eps^2) / cutoff^2 of the 3 att ir^5 term it joins, so it is left out
-  if (s.cutoff > 0.0f && r2 + 1e-12f >= s.unity_r2) {
-    float dist = sqrtf(r2 + 1e-12f);
-    float u = dist / (2.0f * s.cutoff);
-    float e = 1.0f;
-    if (u >= kAttUnityU) {
-      e = expf(-(u * u));
-      att = erfcf(u) + (2.0f / 1.772453850905516f) * u * e;
-    }
-    cc = inv_r3 * dist * e / (2.0f * 1.772453850905516f * s.cutoff * s.cutoff * s.cutoff);
-  }
-  float rg = rx * gx + ry * gy + rz * gz;
-  float lin = att * inv_r3;
-  float rad = rg * (3.0f * att * inv_r5 + cc);
-  ax += -mass * (lin * gx - rad * rx);
-  ay += -mass * (lin * gy - rad * ry);
-  az += -mass * (lin * gz - rad * rz);
-}
-
 // gravityGrad (include/kernel.h:89-94): -m / (|r| + 0.1)^3 * r.
 __device__ __forceinline__ float grav_grad_coeff(float r2, float mass) {
   float dist = sqrtf(r2);

@@ -6,10 +6,10 @@
 // prune radius (the short range of TreePM), and a quadrupole radius beyond
 // which accepted nodes keep the monopole alone.
 //
-// Traversal: one warp per target group of at most kGroup targets (kTPL per
-// lane), cut from the tree so its box is compact; every opening decision is
-// taken on the group's box, so it is warp-uniform; warps take groups from an
-// atomic counter (persistent grid).
+// Traversal: the warps of a block share one target group of at most kGroup
+// targets (kTPL per lane), cut from the tree so its box is compact; every
+// opening decision is taken on the group's box, one node per lane; blocks take
+// groups from an atomic counter (persistent grid).
 //
 // Tree definition (the CPU oracle restates it; integer fields are pinned
 // bit-exactly):
@@ -602,7 +602,7 @@ struct WalkTree {
 struct WalkTargets {
   const float4* tp;          // sorted target positions
   const uint32_t* perm;      // sorted slot -> input index
-  const int4* groups;        // (start, end, system, 0), <= 32 targets each
+  const int4* groups;        // (start, end, system, 0), <= kGroup targets each
   const uint32_t* ngroups;   // device-side group count
   int self;                  // targets are the sources (skip i == j pairs)
   uint32_t* counter;         // work counter, zero at launch
@@ -610,10 +610,10 @@ struct WalkTargets {
   int64_t tbeg, tend;        // groups whose first sorted target lies outside [tbeg, tend) are skipped
 };
 
-// Persistent walks: the grid holds as many warps as the SMs keep resident,
-// and each warp takes its next group from an atomic counter until none is
-// left, so a warp that drew cheap groups keeps working while another is
-// still on an expensive one (group costs in one tree differ by 10x and
+// Persistent walks: the grid holds as many blocks as the SMs keep resident,
+// and each block (coop_next_group; in the count-only walk each warp) takes its
+// next group from an atomic counter until none is left, so a block that drew
+// cheap groups keeps working while another is still on an expensive one (group costs in one tree differ by 10x and
 // more between the core and the halo of a clustered distribution).
 __device__ __forceinline__ uint32_t next_group(const WalkTargets& G) {
   uint32_t s = 0;
@@ -1641,7 +1641,7 @@ WalkTargets self_targets(const Layout& L, const Header& h) {
 bool partial_range(const Header& h) { return h.tbeg > 0 || h.tend < h.n; }
 
 // Blocks of a persistent walk: resident blocks per SM x SMs, and no more
-// than one warp per possible group. Occupancy is queried per kernel and
+// than the possible groups need. Occupancy is queried per kernel and
 // device once (a host-side query; nothing is enqueued).
 template <typename K>
 unsigned walk_blocks(K kernel, int64_t max_groups, int per_block = 4, int threads = 128, size_t smem = 0) {

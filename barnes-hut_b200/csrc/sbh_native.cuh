@@ -13,7 +13,7 @@ struct SegBox {
   double scale;  // 2^21 / span
 };
 
-// One node, 64 bytes, read by the traversal with four 16-byte loads.
+// One node, 80 bytes, read by the traversal with 16-byte loads.
 struct NodeRec {
   float4 com;    // COM x, y, z and total mass M
   float4 cell;   // cell centre x, y, z and diag = side * sqrt(3)
@@ -24,11 +24,11 @@ struct NodeRec {
 static_assert(sizeof(NodeRec) == 80, "NodeRec must be 80 bytes");
 
 constexpr int kLeafFlag = 0x100;
-// Most targets per group: four per lane of a warp. Groups of at most
+// Most targets per group: four per lane, in every warp of the block. Groups of at most
 // kGroupTwoSlots targets are walked by the two-slot kernels, larger ones by the
 // four-slot kernels.
 constexpr int kGroupTwoSlots = 64;
-constexpr int kGroup = 128;  // targets per group built by default (one warp, four per lane)
+constexpr int kGroup = 128;  // targets per group built by default (four per lane)
 #ifndef SBH_QUERY_GROUP
 #define SBH_QUERY_GROUP 32
 #endif

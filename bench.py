@@ -1191,11 +1191,11 @@ WALK_LAUNCHES = 2
 
 # DRAM bytes (read + write) of one adjoint walk per particle, from one ncu
 # capture (dram__bytes_read.sum + dram__bytes_write.sum) of the packed walk
-# (four targets per lane, node tiles, linearized quadrupoles) over 4 Plummer
-# systems of 262,144 particles: 127.01 MB + 39.26 MB for 1,048,576 particles.
+# (four targets per lane, four warps per group, linearized quadrupoles) over 4
+# Plummer systems of 262,144 particles: 137.19 MB + 42.88 MB for 1,048,576.
 # The walk's DRAM traffic is its L2 misses on the tree, the particles and the
 # adjoint arrays, which grow with the particle count.
-WALK_DRAM_BYTES_PER_PARTICLE = 158.6
+WALK_DRAM_BYTES_PER_PARTICLE = 171.7
 FINALIZE_LAUNCHES = 5
 
 # FP32 flops of the adjoint walk (force + adjoint, counted from
@@ -1226,9 +1226,9 @@ BUILD_ALG_BYTES_PER_PARTICLE = 16 + 20
 BUILD_ALG_BYTES_PER_NODE = 80
 
 # DRAM bytes (read + write) of one forest build per particle, summed over the
-# build's 69 kernels from one ncu capture of the bench's 8 x 2^20 Plummer
-# forest (4,911.9 MB read + 1,900.0 MB written).
-BUILD_DRAM_BYTES_PER_PARTICLE = 812.0
+# build's 68 kernels from one ncu capture of the bench's 8 x 2^20 Plummer
+# forest (4,419.2 MB read + 1,453.5 MB written).
+BUILD_DRAM_BYTES_PER_PARTICLE = 700.0
 
 
 def hbm_peak_gbs():

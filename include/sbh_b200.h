@@ -387,7 +387,7 @@ typedef struct sbh_native_params {
                               group instead of one per target; 0: every quadrupole is exact */
 } sbh_native_params;
 
-/* Most targets one group holds (one warp walks a group). */
+/* Most targets one group holds (a lane of the walk holds four). */
 int sbh_native_group_size(void);
 
 /* Forgets the tree recorded for `workspace` in the host registry (sizes,
