@@ -399,8 +399,9 @@ __device__ __forceinline__ bool o8_unity(float r2, const Soft& s) {
   return !(s.cutoff > 0.0f && o8_add(r2, 1e-12f) >= s.unity_r2);
 }
 
-// erfc attenuation of one pair outside the att = 1 range (soft_coeff's and
-// soft_vjp_accum's slow path): att, and the VJP's radial term cc.
+// erfc attenuation of one pair outside the att = 1 range (soft_coeff's slow
+// path): att, and the VJP's radial term cc. Within that range cc stays below
+// 1e-4 (r^2 + eps^2) / cutoff^2 of the 3 att ir^5 term it joins and is left out.
 __device__ __forceinline__ void o8_soft_att(float r2, float ir3, const Soft& s, float& att, float& cc) {
   float dist = sqrtf(o8_add(r2, 1e-12f));
   float u = dist / (2.0f * s.cutoff);
@@ -1030,8 +1031,18 @@ struct O8UnitSums {
   int next;
 };
 
+// Blocks of 128 threads per SM with own query sets: 6 (80 registers) for the
+// forces; the VJPs 7 (72), in a periodic box 8 (64), so that trees of 10^6
+// particles, where more warps hide more of the visits' latency, are not slower
+// than without the prefetch: Plummer 218 ms against 225 at 6 blocks (222 without
+// prefetch), periodic 8.06 against 8.34 (8.00). It costs a VJP 4% at 60,000 to
+// 100,000 particles (6.8 and 8.6 ms; 8.4 and 10.6 without prefetch). Forces at 7
+// blocks: 153 ms against 149 at 10^6.
+template <int KERNEL, bool STAGED>
+constexpr int kO8OwnBlocks = KERNEL == O8_SOFT_VJP || KERNEL == O8_GRAV_GRAD_VJP ? (STAGED ? 7 : 8) : 6;
+
 template <int KERNEL, int STACK, bool STAGED, int WQ>
-__global__ void __launch_bounds__(256, 3)
+__global__ void __launch_bounds__(WQ > 1 ? 256 : 128, WQ > 1 ? 3 : kO8OwnBlocks<KERNEL, STAGED>)
     o8_bh_warp_kernel(const Leaf3* __restrict__ leaf, const OctreeNode8* __restrict__ nodes,
                       const float* __restrict__ queries, const float* __restrict__ cot, int64_t nq, float beta,
                       Soft s, int prune_on, float r_cut_sq, Periodic per, float* __restrict__ out, uint32_t* status,
