@@ -827,7 +827,7 @@ struct WalkQueues {
   int quad[64 * W];   // accepted nodes with the exact quadrupole
   int2 leaf[64 * W];  // near leaves: first particle, count
   int4 cnt[W];        // one step's additions per warp (far, quad, leaf, stack)
-  float box[12];      // group box: minima, maxima; its centre and squared half diagonal
+  float box[16];      // group box: minima, maxima; centre, squared half diagonal; centre in its frame, frame
   uint32_t group;
 };
 
@@ -841,6 +841,8 @@ struct WalkTags {
 // One warp's share: the staged sources of its batch, their indices, its sums
 // of the linearized quadrupoles (a_q (3), J (6) per lane) and, for the
 // adjoint, the group's cotangent sums (W (3), V (6)) and the reduction buffer.
+enum { kNoImage = 0, kShifted = 1, kOwnImage = 2 };  // periodic batches (group_image)
+constexpr int kStageLow = 64;  // a shifted batch's low parts, behind its 32 splatted sources
 constexpr int kRedStride = 36;  // float4 per row: 32 lanes, padded so four lanes' reads of eight rows miss each other's banks
 template <bool ADJ>
 struct WarpShared {
@@ -1012,10 +1014,14 @@ __device__ __forceinline__ int leaf_particle(const LeafShare& s, int b, int lane
   return b + lane < s.total ? start + b + lane - excl : -1;
 }
 
-// The group's box into shared memory and its root onto the stack.
+// The group's box into shared memory and its root onto the stack. A periodic walk
+// (L: the box length, else 0) takes the pairs of a group in the last quarter of
+// [0, L] one box lower: those targets, and the sources of the box's upper half,
+// move there without rounding (x - L for L/2 <= x <= 2 L), and the sources across
+// the boundary, which would round in x + L, stay.
 template <int W>
 __device__ __forceinline__ void coop_begin(WalkQueues<W>& q, const float* gmin, const float* gmax, const int2& root,
-                                           int warp, int lane) {
+                                           int warp, int lane, float L = 0.0f) {
   if (warp == 0 && lane == 0) {
     float c4[4];
     lq_group_centre(gmin, gmax, c4);
@@ -1026,6 +1032,12 @@ __device__ __forceinline__ void coop_begin(WalkQueues<W>& q, const float* gmin, 
     }
 #pragma unroll
     for (int d = 0; d < 4; d++) q.box[6 + d] = c4[d];
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      const float f = gmin[d] >= 0.75f * L && gmax[d] <= 1.25f * L ? -L : 0.0f;
+      q.box[10 + d] = c4[d] + f;
+      q.box[13 + d] = f;
+    }
     q.stack[0] = root.x;
   }
   __syncthreads();
