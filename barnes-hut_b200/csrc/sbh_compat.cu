@@ -979,7 +979,7 @@ __global__ void __launch_bounds__(256)
 // WQ = 8: the block's eight warps share one set of 32 queries. Every warp walks
 // the tree's top two levels and takes units (O8Units) off a counter; the units'
 // sums meet in shared memory and are added in order. WQ = 1: each warp of the
-// block has its own queries.
+// block has its own `per_set` queries (the lanes past them idle).
 // The block's dynamic shared memory holds each warp's leaf buffer (32 x 16 B),
 // then each warp's stack of STACK entries (64 for a dense octree8 of depth <= 9:
 // a DFS of depth d holds at most 7 d + 1 entries; otherwise the reference's
@@ -1046,7 +1046,7 @@ __global__ void __launch_bounds__(WQ > 1 ? 256 : 128, WQ > 1 ? 3 : kO8OwnBlocks<
     o8_bh_warp_kernel(const Leaf3* __restrict__ leaf, const OctreeNode8* __restrict__ nodes,
                       const float* __restrict__ queries, const float* __restrict__ cot, int64_t nq, float beta,
                       Soft s, int prune_on, float r_cut_sq, Periodic per, float* __restrict__ out, uint32_t* status,
-                      O8Bounds bd, const uint32_t* __restrict__ order) {
+                      O8Bounds bd, const uint32_t* __restrict__ order, int per_set) {
   extern __shared__ float4 o8_smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   O8Chunk& chunk = reinterpret_cast<O8Chunk*>(o8_smem)[warp];
@@ -1056,8 +1056,8 @@ __global__ void __launch_bounds__(WQ > 1 ? 256 : 128, WQ > 1 ? 3 : kO8OwnBlocks<
                                                     o8_warp_smem(static_cast<int>(blockDim.x >> 5), STACK));
   const int64_t set = WQ > 1 ? static_cast<int64_t>(blockIdx.x)
                              : static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + warp;
-  const int64_t ti = set * 32 + lane;
-  const bool valid = ti < nq;
+  const int64_t ti = set * per_set + lane;
+  const bool valid = lane < per_set && ti < nq;
   const uint32_t live = __ballot_sync(0xffffffffu, valid);
   if (live == 0) return;  // uniform over the warps of a set
   int mine = 0;           // WQ > 1: the unit this warp takes next
@@ -1615,19 +1615,19 @@ static bool o8_small_stack(uint32_t num_nodes) {
 // straight from global memory and holds fewer registers (TreePM short range,
 // 2^21 particles: 16.6 ms against 17.7 ms staged).
 template <int KERNEL, int STACK, int WQ>
-static void o8_launch_warp_kind(int warps, cudaStream_t stream, const Leaf3* L, const OctreeNode8* N,
+static void o8_launch_warp_kind(int warps, int per_set, cudaStream_t stream, const Leaf3* L, const OctreeNode8* N,
                                 const float* queries, const float* cot, int64_t nq, float beta, Soft s, int prune_on,
                                 float r_cut_sq, Periodic per, float* out, uint32_t* status, O8Bounds bd,
                                 const uint32_t* order) {
   const unsigned block = 32u * static_cast<unsigned>(warps);
-  const unsigned grid = grid_for(nq, WQ > 1 ? 32 : static_cast<int>(block));
+  const unsigned grid = grid_for(nq, WQ > 1 ? per_set : per_set * warps);
   const size_t smem = o8_warp_smem(warps, STACK) + (WQ > 1 ? sizeof(O8UnitSums) : 0);
   if (per.on)
     o8_bh_warp_kernel<KERNEL, STACK, false, WQ><<<grid, block, smem, stream>>>(
-        L, N, queries, cot, nq, beta, s, prune_on, r_cut_sq, per, out, status, bd, order);
+        L, N, queries, cot, nq, beta, s, prune_on, r_cut_sq, per, out, status, bd, order, per_set);
   else
     o8_bh_warp_kernel<KERNEL, STACK, true, WQ><<<grid, block, smem, stream>>>(
-        L, N, queries, cot, nq, beta, s, prune_on, r_cut_sq, per, out, status, bd, order);
+        L, N, queries, cot, nq, beta, s, prune_on, r_cut_sq, per, out, status, bd, order, per_set);
 }
 
 // Eight warps share 32 queries while the query sets alone give the SMs fewer
@@ -1641,13 +1641,24 @@ static void o8_launch_warp_kind(int warps, cudaStream_t stream, const Leaf3* L, 
 // sphere 7.2 / 7.5 and 6.3 / 6.8; 10^5 12.5 / 13.2 and 8.5 / 9.7 (9.6 / 10.7 before).
 static bool o8_shared_sets(int64_t nq, uint32_t leaves) { return nq <= 148 * 16 * 32 && leaves <= kO8UnitLeaves; }
 
+// Queries per warp that walks them down one stack. The 32 of a warp share visits
+// when they are near each other; few queries in a large tree are far apart, and a
+// warp then visits up to 32 queries' nodes one after the other while most of the
+// chip idles. So below 4,096 queries a warp takes one (up to 16 warps per SM), then
+// four. Force, ms on a B200, with 32 per warp / now / one thread per query: 64
+// queries of 2^20 uniform particles 56 / 3.6 / 10, 1,000 41 / 4.0 / 15, 4,095 30 /
+// 9.7 / 15; of a Plummer sphere 48 / 15 / 270, 36 / 16 / 297, 30 / 19 / 315; 64
+// queries of 17,000 uniform particles 11 / 1.9 / 5.0.
+static int o8_queries_per_warp(int64_t nq) { return nq >= 4096 ? 32 : nq > 148 * 16 ? 4 : 1; }
+
 template <int KERNEL, int STACK, typename... A>
 static void o8_launch_warp_sets(int threads, int64_t nq, uint32_t leaves, cudaStream_t stream, A... args) {
   if (o8_shared_sets(nq, leaves)) {
-    o8_launch_warp_kind<KERNEL, STACK, 8>(8, stream, args...);
+    o8_launch_warp_kind<KERNEL, STACK, 8>(8, 32, stream, args...);
   } else {
-    const int warps = threads >= 64 ? (threads < 128 ? threads / 32 : 4) : 1;
-    o8_launch_warp_kind<KERNEL, STACK, 1>(warps, stream, args...);
+    const int per_warp = o8_queries_per_warp(nq);
+    const int warps = threads >= 64 && per_warp == 32 ? (threads < 128 ? threads / 32 : 4) : 1;
+    o8_launch_warp_kind<KERNEL, STACK, 1>(warps, per_warp, stream, args...);
   }
 }
 

@@ -230,10 +230,14 @@ size_t sbh_traversal_workspace_bytes(void);
  * their VJPs and the stochastic ones) of nq queries take the queries in
  * Morton order of their positions: a warp's threads then walk nearby paths,
  * and the deterministic ones walk them down one stack per warp, reading each
- * node once for the lanes that reach it. Every query's result is the same in
- * either order (each query takes its own decisions in its own order, its
+ * node once for the lanes that reach it (below 4,096 queries a warp takes one to
+ * four queries of a tree of more than 16,384 particles). Every query's result is the
+ * same in either order (each query takes its own decisions in its own order, its
  * curand streams seeded by its own index); with a smaller workspace, or
- * below 4,096 queries, they run in input order, one thread per query. */
+ * below 64 queries, they run in input order, one thread per query. In both, a
+ * deterministic traversal of a tree of at most 16,384 particles sums the root, its
+ * children and each of their children's subtrees from zero and adds those sums in
+ * DFS order; of a larger tree all terms join one running sum. */
 size_t sbh_traversal_ordered_workspace_bytes(int64_t nq);
 
 /* ---------------------------------------------------------------------- */
