@@ -635,17 +635,6 @@ struct __align__(16) DirectTile {
   float box[kDirectWarps][8];  // per chunk of 32: minima, maxima
 };
 
-__device__ __forceinline__ float warp_min(float v) {
-  float r;
-  asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
-  return r;
-}
-__device__ __forceinline__ float warp_max(float v) {
-  float r;
-  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
-  return r;
-}
-
 template <bool PER>
 __device__ __forceinline__ float direct_image(float d, float inv_l, const Periodic& per) {
   return PER ? min_image_rint(d, inv_l, per) : d;

@@ -506,14 +506,15 @@ __global__ void roots_kernel(const int64_t* __restrict__ sorted_seg_off, int nse
 // interactions, so the persistent walks hand out the expensive groups first
 // and the cheap ones fill the tail. Within a level the order comes from
 // atomics and varies between runs; each group's result does not.
-constexpr int kGroupBins = 24;  // levels 0..22 (a run of children sits one level below its parent)
+constexpr int kGroupLevels = 24;  // levels 0..22 (a run of children sits one level below its parent)
+constexpr int kGroupBins = 2 * kGroupLevels;  // of the larger systems, then of the small ones
 
 template <bool COUNT>
 __device__ __forceinline__ void emit_chunks(int4* groups, uint32_t* bins, int64_t cap, int s0, int s1, int sys,
-                                            int G, int level, uint32_t* status) {
+                                            int G, int level, bool small, uint32_t* status) {
   int ng = (s1 - s0 + G - 1) / G;
   if (ng <= 0) return;
-  const int bin = kGroupBins - 1 - min(level, kGroupBins - 1);
+  const int bin = (small ? kGroupBins : kGroupLevels) - 1 - min(level, kGroupLevels - 1);
   if (COUNT) {
     atomicAdd(&bins[bin], static_cast<uint32_t>(ng));
     return;
@@ -530,7 +531,8 @@ __device__ __forceinline__ void emit_chunks(int4* groups, uint32_t* bins, int64_
 
 template <bool COUNT>
 __global__ void group_nodes_kernel(const NodeRec* __restrict__ nodes, const uint32_t* __restrict__ nn_ptr,
-                                   const uint32_t* __restrict__ sseg, int4* __restrict__ groups, int64_t cap, int G,
+                                   const uint32_t* __restrict__ sseg, const int64_t* __restrict__ seg_off,
+                                   int64_t alone, int4* __restrict__ groups, int64_t cap, int G,
                                    uint32_t* __restrict__ bins, uint32_t* status) {
   uint32_t nn = *nn_ptr;
   for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += gridDim.x * blockDim.x) {
@@ -540,15 +542,16 @@ __global__ void group_nodes_kernel(const NodeRec* __restrict__ nodes, const uint
     int level = t.w & 0xFF;
     bool root = level == 0;
     int sys = sseg ? static_cast<int>(sseg[t.x]) : 0;
+    const bool small = sseg && seg_off[sys + 1] - seg_off[sys] <= alone;
     if (leaf || cnt <= G) {
-      if (root || (leaf && cnt > G)) emit_chunks<COUNT>(groups, bins, cap, t.x, t.y, sys, G, level, status);
+      if (root || (leaf && cnt > G)) emit_chunks<COUNT>(groups, bins, cap, t.x, t.y, sys, G, level, small, status);
       continue;
     }
     int run_s = -1, run_e = -1;
     for (uint32_t c = k + 1; c < static_cast<uint32_t>(t.z) && c < nn;) {
       int4 tc = nodes[c].topo;
       if (tc.y - tc.x > G) {
-        if (run_s >= 0) emit_chunks<COUNT>(groups, bins, cap, run_s, run_e, sys, G, level + 1, status);
+        if (run_s >= 0) emit_chunks<COUNT>(groups, bins, cap, run_s, run_e, sys, G, level + 1, small, status);
         run_s = -1;
       } else {
         if (run_s < 0) run_s = tc.x;
@@ -557,16 +560,17 @@ __global__ void group_nodes_kernel(const NodeRec* __restrict__ nodes, const uint
       if (static_cast<uint32_t>(tc.z) <= c) break;  // malformed skip: never loop
       c = static_cast<uint32_t>(tc.z);
     }
-    if (run_s >= 0) emit_chunks<COUNT>(groups, bins, cap, run_s, run_e, sys, G, level + 1, status);
+    if (run_s >= 0) emit_chunks<COUNT>(groups, bins, cap, run_s, run_e, sys, G, level + 1, small, status);
   }
 }
 
-// Tallies per level -> cursors (exclusive offsets, deepest level first) and
-// the group count.
-__global__ void group_bins_kernel(uint32_t* bins, uint32_t* group_count) {
+// Tallies per level -> cursors (exclusive offsets, deepest level first), the
+// group count and where the small systems' groups begin.
+__global__ void group_bins_kernel(uint32_t* bins, uint32_t* group_count, uint32_t* small_begin) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   uint32_t run = 0;
   for (int b = 0; b < kGroupBins; b++) {
+    if (b == kGroupLevels) *small_begin = run;
     uint32_t c = bins[b];
     bins[b] = run;
     run += c;
@@ -603,7 +607,8 @@ struct WalkTargets {
   const float4* tp;          // sorted target positions
   const uint32_t* perm;      // sorted slot -> input index
   const int4* groups;        // (start, end, system, 0), <= kGroup targets each
-  const uint32_t* ngroups;   // device-side group count
+  const uint32_t* ngroups;   // device-side end of the groups
+  const uint32_t* first;     // device-side first of them (null: 0)
   int self;                  // targets are the sources (skip i == j pairs)
   uint32_t* counter;         // work counter, zero at launch
   uint32_t capacity;         // entries of groups (bounds the device-side count)
@@ -868,12 +873,17 @@ struct __align__(16) CoopShared {
 
 template <int W>
 __device__ __forceinline__ uint32_t coop_next_group(const WalkTargets& G, WalkQueues<W>& q) {
-  if (threadIdx.x == 0) q.group = atomicAdd(G.counter, 1u);
+  if (threadIdx.x == 0) q.group = atomicAdd(G.counter, 1u) + (G.first ? *G.first : 0u);
   __syncthreads();
   const uint32_t gw = q.group;
   __syncthreads();
   return gw;
 }
+
+// The launch for a forest's small systems (launch_part) may fill the chip as the
+// one before it runs out of groups, and ends after it.
+__device__ __forceinline__ void launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // The walk's state, the same in every warp of the group.
 struct Frontier {
@@ -1339,7 +1349,7 @@ struct Layout {
   int2* roots;
   int4* groups;
   uint32_t* work;  // persistent-walk work counters
-  uint32_t* meta;  // [0] node count, [1] group count, [2] which ping-pong buffer holds perm
+  uint32_t* meta;  // [0] node count, [1] group count, [3] nodes over capacity, [4] first group of a small system
   uint32_t* gbins;  // per-level group tallies, then cursors (group_nodes_kernel)
   unsigned long long* counters;
   // adjoint scratch
@@ -1463,19 +1473,50 @@ namespace {
 std::mutex g_reg_mu;
 std::unordered_map<const void*, Header> g_registry;
 
-// Target groups of at most G targets, deepest cells first (group_nodes_kernel).
+// Warps per group: 16 while the groups (estimated as three quarters full) are
+// fewer than 12 per SM, else 4. Force / force + adjoint in ms on a B200 with 4
+// and 16 warps: Plummer spheres of 10^4 particles (groups of 128) 0.43 / 0.91
+// and 0.14 / 0.38, 10^5 2.02 / 4.63 and 1.49 / 3.74, 2 x 10^5 2.13 / 4.81 and
+// 2.31 / 5.01, 4 x 10^5 3.77 / 9.00 and 4.26 / 9.80; a uniform cube of 10^5 in
+// groups of 64 0.53 / 1.39 and 0.72 / 1.51. Eight warps lie between the two
+// everywhere but at 10^5, where they are within 5% of the better.
+bool coop_wide(int64_t n, int nseg, int G) { return n * 4 / (G * 3) + nseg <= 12 * 148; }
+
+// The most particles of a forest's system whose groups are served by one warp
+// each, in a launch of their own (0: no such launch). Several warps only add
+// barriers to a small system's walk: of many systems, those of up to kAloneMany
+// particles fill the chip with one warp per group; while the groups are fewer than 24
+// per SM only those of up to kAloneFew, about one group, do; and up to 512 systems
+// do not repay a second launch. Force / force + adjoint / stochastic
+// estimate / its VJP in ms on a B200, with 4 warps (8 in the estimates) and one: 10,000
+// systems of 100 particles 0.17 / 0.64 / 0.30 / 1.10 and 0.10 / 0.50 / 0.11 / 0.60, 2,000
+// of 1,000 1.54 / 4.30 / 2.90 / 8.90 and 1.20 / 3.91 / 1.45 / 6.43, 1,000 of 2,000 1.76 /
+// 4.96 / 2.83 / 9.06 and 1.73 / 5.21 / 1.98 / 7.93; 1,000 of 300 0.093 / 0.30 / 0.16 / 0.50
+// and 0.092 / 0.30 / 0.10 / 0.39, of 100 0.042 / 0.13 / 0.05 / 0.17 and 0.043 / 0.14 / 0.04 /
+// 0.15; with 16 warps (8) and one: 1,000 of 30 0.062 / 0.127 / 0.042 / 0.122 and 0.026 /
+// 0.084 / 0.029 / 0.094, 300 of 100 0.042 / 0.106 / 0.036 / 0.109 and 0.037 / 0.116 /
+// 0.046 / 0.138.
+constexpr int kAloneSystems = 512;
+constexpr int64_t kAloneFew = 64, kAloneMany = 1536;
+int64_t alone_max(int64_t n, int nseg, int G) {
+  return nseg <= kAloneSystems ? 0 : n * 4 / (G * 3) + nseg <= 24 * 148 ? kAloneFew : kAloneMany;
+}
+
+// Target groups of at most G targets, deepest cells first (group_nodes_kernel),
+// those of small systems behind the others.
 // `zeroed`: gbins is zero already.
 cudaError_t cut_groups(cudaStream_t stream, const Layout& L, int64_t n, int nseg, int G, uint32_t* status,
                        bool zeroed) {
+  const int64_t alone = alone_max(n, nseg, G);
   cudaError_t e = zeroed ? cudaSuccess : cudaMemsetAsync(L.gbins, 0, kGroupBins * sizeof(uint32_t), stream);
   if (e != cudaSuccess) return e;
   const unsigned grid = gs(static_cast<int64_t>(L.cap));
   const uint32_t* sseg = nseg > 1 ? L.sseg : nullptr;
-  group_nodes_kernel<true><<<grid, 256, 0, stream>>>(L.nodes, L.meta, sseg, L.groups, n + nseg + 1, G, L.gbins,
-                                                     status);
-  group_bins_kernel<<<1, 32, 0, stream>>>(L.gbins, L.meta + 1);
-  group_nodes_kernel<false><<<grid, 256, 0, stream>>>(L.nodes, L.meta, sseg, L.groups, n + nseg + 1, G, L.gbins,
-                                                      status);
+  group_nodes_kernel<true><<<grid, 256, 0, stream>>>(L.nodes, L.meta, sseg, L.seg_off, alone, L.groups,
+                                                     n + nseg + 1, G, L.gbins, status);
+  group_bins_kernel<<<1, 32, 0, stream>>>(L.gbins, L.meta + 1, L.meta + 4);
+  group_nodes_kernel<false><<<grid, 256, 0, stream>>>(L.nodes, L.meta, sseg, L.seg_off, alone, L.groups,
+                                                      n + nseg + 1, G, L.gbins, status);
   return cudaGetLastError();
 }
 
@@ -1646,7 +1687,7 @@ __global__ void zero_node_adj_kernel(float* adj, const uint32_t* meta) {
 WalkTree tree_view(const Layout& L) { return WalkTree{L.nodes, L.child, L.sp, L.sn, L.nnrm, L.roots}; }
 
 WalkTargets self_targets(const Layout& L, const Header& h) {
-  return WalkTargets{L.sp,      L.v0, L.groups, L.meta + 1, 1, L.work, static_cast<uint32_t>(h.n + h.nseg + 1),
+  return WalkTargets{L.sp, L.v0, L.groups, L.meta + 1, nullptr, 1, L.work, static_cast<uint32_t>(h.n + h.nseg + 1),
                      h.tbeg, h.tend};
 }
 
@@ -1699,50 +1740,63 @@ cudaError_t launch_walk(cudaStream_t stream, uint32_t* counter, int64_t max_grou
   return cudaGetLastError();
 }
 
-// A walk by blocks of W warps, one group at a time.
-template <int W, bool ADJ, typename K, typename... A>
-cudaError_t launch_coop(cudaStream_t stream, uint32_t* counter, int64_t max_groups, K kernel, A... args) {
-  cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(uint32_t), stream);
-  if (e != cudaSuccess) return e;
-  constexpr size_t kSmem = sizeof(CoopShared<W, ADJ>);
-  const unsigned blocks = walk_blocks(kernel, max_groups, 1, 32 * W, kSmem);
-  kernel<<<blocks, 32 * W, kSmem, stream>>>(args...);
-  return cudaGetLastError();
+// A walk by blocks of W warps, one group at a time: the groups of a forest's small
+// systems for W = 1, the others else (nothing when there can be none). The two
+// launches overlap: the second need not wait for the last groups of the first.
+template <int W, typename S, typename... P, typename... A>
+cudaError_t launch_part(cudaStream_t stream, const Layout& L, const Header& h, void (*kernel)(P...), A... args) {
+  const int64_t alone = alone_max(h.n, h.nseg, h.group_size);
+  const bool others = h.n > alone;
+  if (W == 1 ? alone == 0 : !others) return cudaSuccess;
+  WalkTargets G = self_targets(L, h);
+  if (W == 1) {
+    G.first = L.meta + 4;
+    G.counter = L.work + 1;
+  } else if (alone > 0) {
+    G.ngroups = L.meta + 4;
+  }
+  cudaLaunchAttribute overlap{};
+  overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  overlap.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3(walk_blocks(kernel, h.n + h.nseg, 1, 32 * W, sizeof(S)));
+  c.blockDim = dim3(32 * W);
+  c.dynamicSmemBytes = sizeof(S);
+  c.stream = stream;
+  c.attrs = &overlap;
+  c.numAttrs = W == 1 && others ? 1 : 0;
+  return cudaLaunchKernelEx(&c, kernel, tree_view(L), G, args...);
 }
 
 template <bool ADJ>
 cudaError_t launch_stochastic(cudaStream_t stream, const Layout& L, const Header& h, float beta_c, float beta_f,
                               float eps2, int samples, uint64_t seed, const float* cot, float* out) {
-  cudaError_t e = cudaMemsetAsync(L.work, 0, sizeof(uint32_t), stream);
-  if (e != cudaSuccess) return e;
-  constexpr size_t kSmem = sizeof(StochShared<ADJ>);
-  const unsigned blocks = walk_blocks(stoch_kernel<ADJ>, h.n + h.nseg, 1, 32 * kStochWarps, kSmem);
-  stoch_kernel<ADJ><<<blocks, 32 * kStochWarps, kSmem, stream>>>(tree_view(L), self_targets(L, h), beta_c, beta_f, eps2,
-                                                                 samples, seed, cot, out, L.gq, L.node_adj,
-                                                                 L.part_adj);
-  return cudaGetLastError();
+  cudaError_t e = cudaMemsetAsync(L.work, 0, 2 * sizeof(uint32_t), stream);
+  if (e == cudaSuccess)
+    e = launch_part<8, StochShared<ADJ, 8>>(stream, L, h, stoch_kernel<ADJ, 8>, beta_c, beta_f, eps2, samples,
+                                                 seed, cot, out, L.gq, L.node_adj, L.part_adj);
+  if (e == cudaSuccess)
+    e = launch_part<1, StochShared<ADJ, 1>>(stream, L, h, stoch_kernel<ADJ, 1>, beta_c, beta_f, eps2, samples,
+                                                 seed, cot, out, L.gq, L.node_adj, L.part_adj);
+  return e;
 }
 
 #define SBH_NT_LAUNCH_W(W, ADJ, KERNEL, ...)                                                                    \
-  launch_coop<W, ADJ>(stream, L.work, h.n + h.nseg,                                                             \
-                      h.group_size > kGroupTwoSlots                                                             \
-                          ? SBH_NT_SELECT_W(tpl4, KERNEL, W, params->quadrupole, params->periodic != 0,         \
-                                            params->cutoff > 0.0f)                                              \
-                          : SBH_NT_SELECT_W(tpl2, KERNEL, W, params->quadrupole, params->periodic != 0,         \
-                                            params->cutoff > 0.0f),                                             \
-                      __VA_ARGS__)
-#define SBH_NT_LAUNCH_COOP(ADJ, KERNEL, ...)                       \
-  e = coop_wide(h) ? SBH_NT_LAUNCH_W(16, ADJ, KERNEL, __VA_ARGS__) \
-                   : SBH_NT_LAUNCH_W(4, ADJ, KERNEL, __VA_ARGS__)
-
-// Warps per group: 16 while the groups (estimated as three quarters full) are
-// fewer than 12 per SM, else 4. Force / force + adjoint in ms on a B200 with 4
-// and 16 warps: Plummer spheres of 10^4 particles (groups of 128) 0.43 / 0.91
-// and 0.14 / 0.38, 10^5 2.02 / 4.63 and 1.49 / 3.74, 2 x 10^5 2.13 / 4.81 and
-// 2.31 / 5.01, 4 x 10^5 3.77 / 9.00 and 4.26 / 9.80; a uniform cube of 10^5 in
-// groups of 64 0.53 / 1.39 and 0.72 / 1.51. Eight warps lie between the two
-// everywhere but at 10^5, where they are within 5% of the better.
-bool coop_wide(const Header& h) { return h.n * 4 / (h.group_size * 3) + h.nseg <= 12 * 148; }
+  launch_part<W, CoopShared<W, ADJ>>(stream, L, h,                                                         \
+                                          h.group_size > kGroupTwoSlots                                         \
+                                              ? SBH_NT_SELECT_W(tpl4, KERNEL, W, params->quadrupole,            \
+                                                                params->periodic != 0, params->cutoff > 0.0f)   \
+                                              : SBH_NT_SELECT_W(tpl2, KERNEL, W, params->quadrupole,            \
+                                                                params->periodic != 0, params->cutoff > 0.0f),  \
+                                          __VA_ARGS__)
+#define SBH_NT_LAUNCH_COOP(ADJ, KERNEL, ...)                                                              \
+  {                                                                                                       \
+    e = cudaMemsetAsync(L.work, 0, 2 * sizeof(uint32_t), stream);                                         \
+    if (e == cudaSuccess)                                                                                 \
+      e = coop_wide(h.n, h.nseg, h.group_size) ? SBH_NT_LAUNCH_W(16, ADJ, KERNEL, __VA_ARGS__)            \
+                                               : SBH_NT_LAUNCH_W(4, ADJ, KERNEL, __VA_ARGS__);            \
+    if (e == cudaSuccess) e = SBH_NT_LAUNCH_W(1, ADJ, KERNEL, __VA_ARGS__);                               \
+  }
 
 int check_params(const sbh_native_params* p) {
   if (!p) return invalid("params must be non-null");
@@ -1859,7 +1913,7 @@ int sbh_native_force(cudaStream_t stream, const sbh_native_params* params, float
   if (partial_range(h)) e = cudaMemsetAsync(force_out, 0, h.n * 3 * sizeof(float), stream);
   if (e != cudaSuccess) return fail(SBH_ERR_CUDA, cudaGetErrorString(e));
   WalkParams wp = walk_params(params);
-  SBH_NT_LAUNCH_COOP(false, force_walk_kernel, tree_view(L), self_targets(L, h), wp, force_out);
+  SBH_NT_LAUNCH_COOP(false, force_walk_kernel, wp, force_out)
   if (e != cudaSuccess) return fail(SBH_ERR_CUDA, cudaGetErrorString(e));
   remember_walk(workspace, 1, params);
   return check_launch("sbh_native_force");
@@ -1884,8 +1938,7 @@ int sbh_native_adjoint_walk(cudaStream_t stream, const sbh_native_params* params
   if (e != cudaSuccess) return fail(SBH_ERR_CUDA, cudaGetErrorString(e));
   zero_node_adj_kernel<<<gs(L.cap * kNodeAdj), 256, 0, stream>>>(L.node_adj, L.meta);
   WalkParams wp = walk_params(params);
-  SBH_NT_LAUNCH_COOP(true, adjoint_walk_kernel, tree_view(L), self_targets(L, h), wp, cotangent, force_out, L.gq,
-                     L.node_adj, L.part_adj);
+  SBH_NT_LAUNCH_COOP(true, adjoint_walk_kernel, wp, cotangent, force_out, L.gq, L.node_adj, L.part_adj)
   if (e != cudaSuccess) return fail(SBH_ERR_CUDA, cudaGetErrorString(e));
   remember_walk(workspace, 1, params);
   return check_launch("sbh_native_adjoint_walk");
@@ -2045,7 +2098,7 @@ int sbh_native_winding_number(cudaStream_t stream, float beta, const float* quer
   query_gather_kernel<<<gs(nq), 256, 0, stream>>>(queries, qperm, nq, tp, groups, qmeta);
   e = cudaMemsetAsync(L.counters, 0, kCounters * sizeof(unsigned long long), stream);
   if (e != cudaSuccess) return fail(SBH_ERR_CUDA, cudaGetErrorString(e));
-  WalkTargets G{tp, qperm, groups, qmeta, 0, qmeta + 2, static_cast<uint32_t>(nq / kQueryGroup + 1), 0, INT64_MAX};
+  WalkTargets G{tp, qperm, groups, qmeta, nullptr, 0, qmeta + 2, static_cast<uint32_t>(nq / kQueryGroup + 1), 0, INT64_MAX};
   WalkParams wp{};
   wp.beta = beta;
   e = launch_walk<1>(stream, qmeta + 2, nq / kQueryGroup + 1, wn_walk_kernel, tree_view(L), G, wp, out, L.counters);
@@ -2104,7 +2157,7 @@ int sbh_native_winding_number_vjp(cudaStream_t stream, float beta, const float* 
     if (e != cudaSuccess) return fail(SBH_ERR_CUDA, cudaGetErrorString(e));
     const uint32_t* qperm = which == 0 ? v0 : v1;
     query_gather_kernel<<<gs(nq), 256, 0, stream>>>(queries, qperm, nq, tp, groups, qmeta);
-    WalkTargets G{tp, qperm, groups, qmeta, 0, qmeta + 2, static_cast<uint32_t>(nq / kQueryGroup + 1), 0, INT64_MAX};
+    WalkTargets G{tp, qperm, groups, qmeta, nullptr, 0, qmeta + 2, static_cast<uint32_t>(nq / kQueryGroup + 1), 0, INT64_MAX};
     WalkParams wp{};
     wp.beta = beta;
     e = launch_walk<1>(stream, qmeta + 2, nq / kQueryGroup + 1, wn_adjoint_walk_kernel, tree_view(L), G, wp, cotangent,
