@@ -169,8 +169,12 @@ __global__ void __launch_bounds__(kScanThreads) scan_tile_apply(Load load, int64
   }
 }
 
-// A few tiles in one block and one launch, the running total carried along.
-constexpr int64_t kScanFewTiles = 8;
+// A few tiles in one block and one launch, the running total carried along: for
+// the moment vectors two, a tile of which takes about 8 us there, as long as the
+// two launches saved (8 tiles of 14 doubles: force + adjoint of 4,000 particles 179
+// us, 138 by three launches; build 138 and 115), for words eight.
+template <typename T>
+constexpr int64_t kScanFewTiles = sizeof(T) <= 8 ? 8 : 2;
 template <typename T, typename Load>
 __global__ void __launch_bounds__(kScanThreads) scan_few_tiles(Load load, int64_t n, T* out, int write_total) {
   constexpr int kItems = ScanCfg<T>::kItems;
@@ -207,7 +211,7 @@ template <typename T, typename Load>
 cudaError_t exclusive_scan(cudaStream_t s, Load load, int64_t n, T* out, T* tmp,
                            bool write_total) {
   int64_t nt = scan_tiles<T>(n);
-  if (nt <= kScanFewTiles) {
+  if (nt <= kScanFewTiles<T>) {
     scan_few_tiles<T, Load><<<1, kScanThreads, 0, s>>>(load, n, out, write_total ? 1 : 0);
     return cudaGetLastError();
   }
