@@ -656,7 +656,7 @@ __global__ void __launch_bounds__(32 * kDirectWarps, 2)
   __shared__ float part[SPLIT > 1 ? kDirectWarps : 1][3][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   constexpr int kChunks = kDirectWarps / SPLIT;  // chunks of 32 sources per warp and tile
-  const int slice = warp % SPLIT;
+  const int slice = warp % SPLIT;  // chunks slice, slice + SPLIT, ...: a short tile is shared too
   const int64_t qi = (static_cast<int64_t>(blockIdx.x) * (kDirectWarps / SPLIT) + warp / SPLIT) * 32 + lane;
   const bool active = qi < nq;
   const int64_t ql = active ? qi : nq - 1;
@@ -698,11 +698,11 @@ __global__ void __launch_bounds__(32 * kDirectWarps, 2)
     __syncthreads();
     load(base + kDirectTile + threadIdx.x);  // in flight during this tile's sums
     const int left = static_cast<int>(n - base < kDirectTile ? n - base : kDirectTile);
-    uint32_t unity = 0xffffffffu;  // bit c: chunk slice * kChunks + c lies in the att = 1 range
+    uint32_t unity = 0xffffffffu;  // bit c: chunk c * SPLIT + slice lies in the att = 1 range
     if (s.cutoff > 0.0f) {
       bool u = false;
       if (lane < kChunks) {
-        const float* tb = T.box[slice * kChunks + lane];
+        const float* tb = T.box[lane * SPLIT + slice];
         float R2 = 0.0f;
         for (int d = 0; d < 3; d++) {
           const float span = fmaxf(fabsf(qbox[3 + d] - tb[d]), fabsf(tb[3 + d] - qbox[d]));
@@ -717,7 +717,7 @@ __global__ void __launch_bounds__(32 * kDirectWarps, 2)
     float ax = 0.f, ay = 0.f, az = 0.f;
     F2 AX = f2_pack(0.f, 0.f), AY = AX, AZ = AX;
     for (int c = 0; c < kChunks; c++) {
-      const int j0 = (slice * kChunks + c) * 32;
+      const int j0 = (c * SPLIT + slice) * 32;
       const int cnt = left - j0 < 32 ? left - j0 : 32;
       if (cnt <= 0) break;
       if ((unity >> c) & 1u) {  // sources past the last one carry mass zero
@@ -1475,24 +1475,46 @@ static unsigned grid_for(int64_t n, int threads) {
   return static_cast<unsigned>(b < 1 ? 1 : b);
 }
 
-// The smallest split that gives every SM two blocks (148 x 32 warps): 16 warps
-// per 32 queries up to 37,888 queries, 4 up to 151,552, else 1. A split costs a
-// share of the tile loads per warp (about 60 instructions per tile against 256
-// for 32 unattenuated sources and 1,600 attenuated ones at SPLIT 16). Against one
-// warp per 64 queries over every source (force / VJP, ms on a B200): 4,096 x
-// 4,096 with erfc on nearly every pair 1.46 / 1.61 -> 0.10 / 0.09, 60,000 x 60,000
-// 21.0 / 23.4 -> 12.9 / 16.0, 2^17 x 2^17 61.5 / 73.3 -> 48.2 / 60.0; without
-// attenuation 60,000 x 60,000 2.73 / 4.33 -> 2.52 / 4.19, 2^18 x 2^18 39.1 / 68.7
-// -> 36.8 / 67.1 (1.9e12 pairs/s, bound by the FMA pipe; the attenuated sums by
-// the instructions of erfcf).
+// Warps per 32 queries of a direct sum: 16 while two blocks per SM hold all of
+// them, then 16, 4 or 1, the one with the least
+// estimated time: waves of two blocks per SM (a last wave of at most one block per
+// SM counts half), times the chunks of 32 sources that a warp sums and a quarter
+// for the block itself, times what a split costs in tile loads and shorter loops, by
+// measurement 1.15, 1.1 and 1 (1.03 in a periodic box, where images and erfc
+// dominate). Force / VJP, ms on a B200,
+// against one warp per 64 queries over every source: 4,096 x 4,096 with erfc on
+// nearly every pair 1.46 / 1.61 -> 0.10 / 0.09, 60,000 x 60,000 21.0 / 23.4 -> 12.9 /
+// 16.0 (4 warps). Fixed lines at 37,888 and 151,552 queries left nearly empty last
+// waves, and idle warps on few sources: 5,000 sources x 151,553 queries,
+// periodic, 3.58 / 4.25 with one warp, 2.55 / 3.07 with 16 (3.13 / 3.65 by one query per
+// thread); 100 x 151,552 periodic 0.137 / 0.157 with 4, 0.069 / 0.080 with one.
+static int direct_split(int64_t n, int64_t nq, bool per) {
+  if (nq <= 2 * 148 * 32) return 16;  // all blocks resident at once
+  const int64_t tail = (n % kDirectTile + 31) / 32;  // chunks of the last tile
+  int best = 1;
+  double least = 0.0;
+  for (int split = 1; split <= 16; split *= 4) {
+    const int64_t blocks = (nq * split + kDirectTile - 1) / kDirectTile, rest = blocks % (2 * 148);
+    const double waves = blocks / (2 * 148) + (rest == 0 ? 0.0 : rest <= 148 ? 0.5 : 1.0);
+    const double chunks = n / kDirectTile * (kDirectWarps / split) + (tail + split - 1) / split;
+    const double cost = waves * (chunks + 0.25) * (split == 1 ? 1.0 : per ? 1.03 : split == 4 ? 1.1 : 1.15);
+    if (split == 1 || cost < least) {
+      best = split;
+      least = cost;
+    }
+  }
+  return best;
+}
+
 template <bool VJP, bool PER>
 static void direct_launch(cudaStream_t stream, const float* pts, const float* masses, int64_t n, const float* queries,
                           const float* cot, int64_t nq, float* out, Soft s, Periodic per) {
   constexpr int kThreads = 32 * kDirectWarps;
-  if (nq <= 148 * 32 * 32 / 4) {
+  const int split = direct_split(n, nq, PER);
+  if (split == 16) {
     direct_soft_kernel<16, VJP, PER>
         <<<grid_for(nq, kThreads / 16), kThreads, 0, stream>>>(pts, masses, n, queries, cot, nq, out, s, per);
-  } else if (nq <= 148 * 32 * 32) {
+  } else if (split == 4) {
     direct_soft_kernel<4, VJP, PER>
         <<<grid_for(nq, kThreads / 4), kThreads, 0, stream>>>(pts, masses, n, queries, cot, nq, out, s, per);
   } else {
