@@ -1062,8 +1062,8 @@ __global__ void __launch_bounds__(WQ > 1 ? 256 : 128, WQ > 1 ? 3 : kO8OwnBlocks<
                                                     o8_warp_smem(static_cast<int>(blockDim.x >> 5), STACK));
   const int64_t set = WQ > 1 ? static_cast<int64_t>(blockIdx.x)
                              : static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + warp;
-  const int64_t ti = set * per_set + lane;
-  const bool valid = lane < per_set && ti < nq;
+  const int64_t ti = WQ > 1 ? set * 32 + lane : set * per_set + lane;
+  const bool valid = (WQ > 1 || lane < per_set) && ti < nq;
   const uint32_t live = __ballot_sync(0xffffffffu, valid);
   if (live == 0) return;  // uniform over the warps of a set
   int mine = 0;           // WQ > 1: the unit this warp takes next
