@@ -1483,8 +1483,8 @@ static unsigned grid_for(int64_t n, int threads) {
 // measurement 1.15, 1.1 and 1 (1.03 in a periodic box, where images and erfc
 // dominate). Force / VJP, ms on a B200,
 // against one warp per 64 queries over every source: 4,096 x 4,096 with erfc on
-// nearly every pair 1.46 / 1.61 -> 0.10 / 0.09, 60,000 x 60,000 21.0 / 23.4 -> 12.9 /
-// 16.0 (4 warps). Fixed lines at 37,888 and 151,552 queries left nearly empty last
+// nearly every pair 1.46 / 1.61 -> 0.10 / 0.09, 60,000 x 60,000 21.0 / 23.4 -> 10.6 /
+// 13.0 (12.9 / 16.0 with 4 warps). Fixed lines at 37,888 and 151,552 queries left nearly empty last
 // waves, and idle warps on few sources: 5,000 sources x 151,553 queries,
 // periodic, 3.58 / 4.25 with one warp, 2.55 / 3.07 with 16 (3.13 / 3.65 by one query per
 // thread); 100 x 151,552 periodic 0.137 / 0.157 with 4, 0.069 / 0.080 with one.

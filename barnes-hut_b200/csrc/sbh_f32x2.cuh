@@ -17,9 +17,14 @@ __device__ __forceinline__ float vmul(float a, float b) { return __fmul_rn(a, b)
 __device__ __forceinline__ float2 vmul(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float vadd(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ float2 vadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
-// 1 / sqrt(a) for a normal a (the walks' h = r^2 + eps^2 + 1e-12): rsqrtf
-// without the rescaling of subnormal arguments, which costs a compare and two
-// multiplications around the one special-function instruction.
+// a b, at least 0 and at most 1 (0 for NaN); the packed form is two instructions.
+__device__ __forceinline__ float vmul_sat(float a, float b) { return __saturatef(__fmul_rn(a, b)); }
+__device__ __forceinline__ float2 vmul_sat(float2 a, float2 b) {
+  return make_float2(vmul_sat(a.x, b.x), vmul_sat(a.y, b.y));
+}
+
+// 1 / sqrt(a) for a normal a (the walks' h = r^2 + eps^2 + 1e-12), with the maximum
+// relative error that the PTX manual states for rsqrt.approx.ftz.f32, 2^-22.9.
 __device__ __forceinline__ float vrsqrt(float a) {
   float r;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));

@@ -636,8 +636,8 @@ struct WalkParams {
   float prune_r2;  // > 0: skip nodes whose cell is farther than sqrt(prune_r2) from the group box
   float quad_g;    // > 0: an accepted node takes the quadrupole only when its opening distance^2 is
                    // below quad_g * (beta * diagonal)^2; 0: every accepted node takes it
-  float inv_2cut;  // 1 / (2 cutoff) (cutoff walks)
-  float cc_coef;   // 1 / (2 sqrt(pi) cutoff^3) (cutoff walks)
+  float inv_32cut;  // 1 / (32 cutoff) (cutoff walks)
+  float cc_coef;    // 1 / (2 sqrt(pi) cutoff^3), at most FLT_MAX: times e^{-u^2} = 0 it stays 0 (cutoff walks)
   float quad_lin;  // kappa^2 > 0: accepted quadrupole nodes with r_g^2 <= kappa^2 |c - cell centre|^2 take
                    // the quadrupole to first order about the group centre c; 0: never
 };
@@ -1824,8 +1824,8 @@ WalkParams walk_params(const sbh_native_params* p) {
                     1.0f / box,
                     p->prune_radius * p->prune_radius,
                     qr > 0.0f ? qr * qr : 0.0f,
-                    static_cast<float>(0.5 / c),
-                    static_cast<float>(1.0 / (2.0 * 1.7724538509055160 * c * c * c)),
+                    static_cast<float>(1.0 / (32.0 * c)),
+                    static_cast<float>(fmin(1.0 / (2.0 * 1.7724538509055160 * c * c * c), 3.4028234663852886e38)),
                     p->quadrupole && p->quadrupole_linear > 0.0f ? p->quadrupole_linear * p->quadrupole_linear
                                                                   : 0.0f};
 }
