@@ -1217,9 +1217,9 @@ class _NativeGravity(torch.autograd.Function):
         return gx, gm, None
 
 
-# Candidate block sizes of autotune_octree8 (warps of 32 Morton-ordered
-# queries per block in the warp-cooperative octree8 traversals).
-AUTOTUNE_OCTREE8_THREADS = (64, 128, 256, 512)
+# Candidate block sizes of autotune_octree8: one to four warps of 32
+# Morton-ordered queries per block (larger `threads` take four as well).
+AUTOTUNE_OCTREE8_THREADS = (32, 64, 96, 128)
 
 
 def autotune_octree8(leaf_bytes, node_bytes, queries, *, candidates=AUTOTUNE_OCTREE8_THREADS, reps: int = 2,
@@ -1228,9 +1228,12 @@ def autotune_octree8(leaf_bytes, node_bytes, queries, *, candidates=AUTOTUNE_OCT
     queries: times softened_barnes_hut_force_octree8 (soft_kwargs as its
     keywords) at each candidate `threads` and returns the fastest. The
     warp-cooperative traversal walks 32 Morton-ordered queries per warp with
-    threads / 32 warps per block; its per-warp shared-memory stack holds 64
-    entries for a dense octree8 of depth <= 9 and 128 otherwise. Results do
-    not depend on the block size."""
+    threads / 32 warps per block, at most four; its per-warp shared-memory stack
+    holds 64 entries for a dense octree8 of depth <= 9 and 128 otherwise. It
+    does not read `threads` below 4,096 queries, nor for up to 75,776 queries of
+    a tree of at most 16,384 particles, whose warps share the queries: the
+    candidates then time the same launch. Results do not depend on the block
+    size."""
     dev = _device()
     leaf, node, q = _u8(leaf_bytes, dev), _u8(node_bytes, dev), _f32(queries, dev)
     trials = []
