@@ -860,15 +860,16 @@ __device__ __forceinline__ uint32_t o8_leaf_end(uint32_t start, uint32_t end, co
   return start <= bd.num_leaves ? (end < bd.num_leaves ? end : bd.num_leaves) : start;
 }
 
-// For trees of up to kO8UnitLeaves particles a query's sum is taken in units: the root, each of its children and each of
-// their children with its whole subtree, in the order of the DFS. Every unit is
-// summed from zero and the units are added in order, so warps may share a
-// query's units without changing a bit of its row. (Larger trees keep the single
-// running sum of the reference's traversal: its rounding grows with the tree,
-// and the units' smaller one, though nearer the 64-bit sum, would leave the
-// reference's rows by 2e-5 at 2^18 particles against 2e-6 here.) Which entry starts a unit
-// follows from the stack's heights: the level-1 entries lie below h1, the
-// level-2 entries of the current level-1 node between h1 and h2.
+// For trees of up to kO8UnitLeaves particles a query's sum is taken in units: the
+// root, each of its children and each of their children with its whole subtree, in
+// the order of the DFS. Every unit is summed from zero and the units are added in
+// order, so warps may share a query's units without changing a bit of its row.
+// (Larger trees keep the single running sum of the reference's traversal: its
+// rounding grows with the tree, and the units' smaller one, though nearer the 64-bit
+// sum, would leave the reference's rows by 2e-5 at 2^18 particles against 2e-6
+// here.) Which entry starts a unit follows from the stack's heights: the level-1
+// entries lie below h1, the level-2 entries of the current level-1 node between h1
+// and h2.
 struct O8Units {
   int h1 = 0, h2 = 0;
   bool started = false;
@@ -1699,20 +1700,20 @@ static void o8_launch_warp(int kernel, int threads, cudaStream_t stream, const L
                            const uint32_t* order) {
   switch (kernel) {
     case O8_GRAV_GRAD:
-      o8_launch_warp_sets<O8_GRAV_GRAD, STACK>(threads, nq, bd.num_leaves, stream, L, N, queries, cot, nq, beta, s, 0, 0.f, per, out,
-                                               status, bd, order);
+      o8_launch_warp_sets<O8_GRAV_GRAD, STACK>(threads, nq, bd.num_leaves, stream, L, N, queries, cot, nq, beta, s,
+          0, 0.f, per, out, status, bd, order);
       break;
     case O8_SOFT:
-      o8_launch_warp_sets<O8_SOFT, STACK>(threads, nq, bd.num_leaves, stream, L, N, queries, cot, nq, beta, s, prune_on, r_cut_sq,
-                                          per, out, status, bd, order);
+      o8_launch_warp_sets<O8_SOFT, STACK>(threads, nq, bd.num_leaves, stream, L, N, queries, cot, nq, beta, s,
+          prune_on, r_cut_sq, per, out, status, bd, order);
       break;
     case O8_GRAV_GRAD_VJP:
-      o8_launch_warp_sets<O8_GRAV_GRAD_VJP, STACK>(threads, nq, bd.num_leaves, stream, L, N, queries, cot, nq, beta, s, 0, 0.f, per,
-                                                   out, status, bd, order);
+      o8_launch_warp_sets<O8_GRAV_GRAD_VJP, STACK>(threads, nq, bd.num_leaves, stream, L, N, queries, cot, nq, beta, s,
+          0, 0.f, per, out, status, bd, order);
       break;
     default:
-      o8_launch_warp_sets<O8_SOFT_VJP, STACK>(threads, nq, bd.num_leaves, stream, L, N, queries, cot, nq, beta, s, prune_on, r_cut_sq,
-                                              per, out, status, bd, order);
+      o8_launch_warp_sets<O8_SOFT_VJP, STACK>(threads, nq, bd.num_leaves, stream, L, N, queries, cot, nq, beta, s,
+          prune_on, r_cut_sq, per, out, status, bd, order);
       break;
   }
 }

@@ -848,7 +848,8 @@ struct WalkTags {
 // adjoint, the group's cotangent sums (W (3), V (6)) and the reduction buffer.
 enum { kNoImage = 0, kShifted = 1, kOwnImage = 2 };  // periodic batches (group_image)
 constexpr int kStageLow = 64;  // a shifted batch's low parts, behind its 32 splatted sources
-constexpr int kRedStride = 36;  // float4 per row: 32 lanes, padded so four lanes' reads of eight rows miss each other's banks
+// float4 per row: 32 lanes, padded so that four lanes' reads of eight rows miss each other's banks
+constexpr int kRedStride = 36;
 template <bool ADJ>
 struct WarpShared {
   float4 stage[96];
@@ -1693,6 +1694,11 @@ WalkTargets self_targets(const Layout& L, const Header& h) {
 
 bool partial_range(const Header& h) { return h.tbeg > 0 || h.tend < h.n; }
 
+WalkTargets query_targets(const float4* tp, const uint32_t* perm, const int4* groups, uint32_t* meta, int64_t nq) {
+  return WalkTargets{tp, perm, groups, meta, nullptr, 0, meta + 2, static_cast<uint32_t>(nq / kQueryGroup + 1),
+                     0, INT64_MAX};
+}
+
 // Blocks of a persistent walk: resident blocks per SM x SMs, and no more
 // than the possible groups need. Occupancy is queried per kernel and
 // device once (a host-side query; nothing is enqueued).
@@ -2098,7 +2104,7 @@ int sbh_native_winding_number(cudaStream_t stream, float beta, const float* quer
   query_gather_kernel<<<gs(nq), 256, 0, stream>>>(queries, qperm, nq, tp, groups, qmeta);
   e = cudaMemsetAsync(L.counters, 0, kCounters * sizeof(unsigned long long), stream);
   if (e != cudaSuccess) return fail(SBH_ERR_CUDA, cudaGetErrorString(e));
-  WalkTargets G{tp, qperm, groups, qmeta, nullptr, 0, qmeta + 2, static_cast<uint32_t>(nq / kQueryGroup + 1), 0, INT64_MAX};
+  WalkTargets G = query_targets(tp, qperm, groups, qmeta, nq);
   WalkParams wp{};
   wp.beta = beta;
   e = launch_walk<1>(stream, qmeta + 2, nq / kQueryGroup + 1, wn_walk_kernel, tree_view(L), G, wp, out, L.counters);
@@ -2157,7 +2163,7 @@ int sbh_native_winding_number_vjp(cudaStream_t stream, float beta, const float* 
     if (e != cudaSuccess) return fail(SBH_ERR_CUDA, cudaGetErrorString(e));
     const uint32_t* qperm = which == 0 ? v0 : v1;
     query_gather_kernel<<<gs(nq), 256, 0, stream>>>(queries, qperm, nq, tp, groups, qmeta);
-    WalkTargets G{tp, qperm, groups, qmeta, nullptr, 0, qmeta + 2, static_cast<uint32_t>(nq / kQueryGroup + 1), 0, INT64_MAX};
+    WalkTargets G = query_targets(tp, qperm, groups, qmeta, nq);
     WalkParams wp{};
     wp.beta = beta;
     e = launch_walk<1>(stream, qmeta + 2, nq / kQueryGroup + 1, wn_adjoint_walk_kernel, tree_view(L), G, wp, cotangent,

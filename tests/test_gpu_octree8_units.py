@@ -17,8 +17,10 @@ pytestmark = pytest.mark.gpu
                                         (16384, 300, 6), (16385, 300, 6)])
 def test_rows_do_not_depend_on_how_warps_share_the_tree(cuda, n, nq, depth):
     """The ordered workspace (warps sharing the units of 32 queries) against the
-    small one (one thread per query), bit for bit, and the force against the
-    oracle's FP64 sums of the same decisions."""
+    small one (one thread per query), bit for bit; force and VJP against the oracle's
+    FP64 sums of the same decisions (FP32 sums of at most 16,385 terms: 1e-5), so a
+    unit left out or counted twice shows; the force against the direct sum within
+    the opening error."""
     rng = np.random.default_rng(n)
     p = rng.random((n, 3), dtype=np.float32)
     m = (rng.random(n) + 0.5).astype(np.float32) / n
@@ -43,7 +45,11 @@ def test_rows_do_not_depend_on_how_warps_share_the_tree(cuda, n, nq, depth):
             assert B.read_device_status(ws) == 0
             rows.append((f, g))
         assert torch.equal(rows[0][0], rows[1][0]) and torch.equal(rows[0][1], rows[1][1])
-        if not prune:  # FP32 sums of at most 16,385 terms
+        okw = dict(eps=1e-2, cutoff=cutoff, prune_enabled=bool(prune), prune_r_cut_mult=2.0, periodic=bool(per))
+        for got, kernel, cot in zip(rows[0], (O.KERNEL_SOFT, O.KERNEL_SOFT_VJP), (None, w)):
+            want, _ = O.bh_octree8(leaf.cpu().numpy(), node.cpu().numpy(), q, 2.0, kernel, cot=cot, **okw)
+            assert rel_l2(got.cpu().numpy(), want) < 1e-5
+        if not prune:
             want = O.direct_force_soft(p, m, q, 1e-2, cutoff, False, 1.0)
             assert rel_l2(rows[0][0].cpu().numpy(), want) < (5e-6 if n < 16 else 2e-2)
 

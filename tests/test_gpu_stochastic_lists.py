@@ -12,7 +12,8 @@ from conftest import rel_l2
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n,beta,coarse,samples", [(3000, 2.0, 1.0, 128), (3000, 2.0, 1.0, 129), (3000, 2.0, 0.75, 1024),
+@pytest.mark.parametrize("n,beta,coarse,samples", [(3000, 2.0, 1.0, 128), (3000, 2.0, 1.0, 129),
+                                                   (3000, 2.0, 0.75, 1024),
                                                    (60000, 9.0, 4.0, 32), (60000, 9.0, 4.0, 200)])
 def test_draws_and_cuts_past_the_lists_match_oracle(cuda, n, beta, coarse, samples):
     """Same draws as the oracle's restatement; tolerances as at the usual sizes
