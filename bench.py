@@ -1110,7 +1110,7 @@ def run_ours(args):
                         "counted_by": (f"num_contribs of the reference's CPU evaluateBarnesHut_stackless on "
                                        f"Tree3D<8,1> (leaf 8, beta 2) over {info['sample_queries']} sampled "
                                        "queries of system 0")}
-        launches = args.steps * (build_launches(K) + WALK_LAUNCHES + FINALIZE_LAUNCHES)
+        launches = args.steps * (build_launches(K) + WALK_LAUNCHES + (K > 512) + FINALIZE_LAUNCHES)
         plain_eps = 1000.0 / plain_ms
         line = {
             "metric": METRIC, "value": value, "unit": "evals/s", "n_gpus": world, "steps": args.steps,
@@ -1179,7 +1179,8 @@ def run_ours(args):
 #   pass on the system id (gather 1 + ceil(log2 K / 8) radix passes x 5 +
 #   gathers 2 + system ids 1). (At the bench's sizes: sorts of up to 16,384
 #   keys and scans of a few tiles take one launch.)
-# walk: zero adjoint 1 + walk 1 = 2; finalize: push 1 + scan 3 + combine 1 = 5
+# walk: zero adjoint 1 + walk 1 = 2 (one more for the small systems of a forest of
+#   more than 512); finalize: push 1 + scan 3 + combine 1 = 5
 def build_launches(k: int) -> int:
     if k <= 1:
         return 59
